@@ -29,6 +29,25 @@ int set_error(int status, const char* fmt, ...) __attribute__((format(printf, 2,
     if (!(cond)) return ::rafb200::set_error(RAFB200_INVALID_ARGUMENT, __VA_ARGS__); \
   } while (0)
 
+// Launches `kernel` as a programmatic dependent of the kernel before it on the stream: its blocks
+// may be placed while that kernel's last blocks still run, and must call grid_dependency_wait()
+// before they touch memory that any earlier work on the stream may write or read.
+template <typename... Params, typename... Args>
+inline cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                    Args... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 inline int dtype_size(int dtype) { return dtype == RAFB200_F32 ? 4 : 2; }
 inline bool dtype_valid(int dtype) { return dtype >= RAFB200_F32 && dtype <= RAFB200_BF16; }
 

@@ -1,8 +1,6 @@
-// Chunk-level building blocks shared by the SGD / Adam kernels and the LANS
-// persistent kernel: a block of kBlockThreads threads walks one chunk
-// (<= kChunkElems elements of one tensor) with 16-byte accesses, two vector
-// passes in flight per thread, and falls back to scalar accesses for unaligned
-// tensors and ragged tails.
+// Building blocks of the update kernels: the per-element arithmetic of SGD, Adam and LANS,
+// and the walk of a block over one span of a tensor with 16-byte accesses (scalar ones for
+// unaligned tensors and ragged tails).
 #pragma once
 #include "common.h"
 #include "vec_io.cuh"
@@ -11,7 +9,6 @@ namespace rafb200 {
 
 constexpr int kVec = 4;                              // elements per thread per pass
 constexpr int kPassElems = kBlockThreads * kVec;     // 1024
-constexpr int kUnroll = 2;                           // passes in flight
 constexpr uint32_t kFlagAligned = 1u;  // vector accesses allowed (16 B fp32, 8 B 16-bit arrays)
 constexpr uint32_t kFlagBulk = 2u;     // every array is 16-byte aligned: TMA bulk copies allowed
 
@@ -29,20 +26,105 @@ struct SgdOp {
     p = sub(p, mul(lr, v1));
     m = v1;
   }
+  __device__ __forceinline__ void vec(const F4& g, F4& p, F4& m, F4& v) const {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) (*this)(g.x[j], p.x[j], m.x[j], v.x[j]);
+  }
 };
+
+__device__ __forceinline__ float rcp_approx(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Correctly rounded a/b and sqrt(x) without a branch, for operands far from overflow and
+// underflow (AdamOp::vec checks).  The library forms test every operand and branch, which keeps
+// the elements a thread holds from being interleaved.
+// a/b: P. Markstein, "Computation of elementary functions on the IBM RISC System/6000 processor"
+// (1990): with y = RN(1/b) and q within one unit of a/b, RN(q + RN(a - b*q) * y) is RN(a/b).  The
+// first step brings a*y (up to 1.5 units off) within one unit, the second one rounds.
+__device__ __forceinline__ float div_by(float a, float b, float y) {
+  float q = mul(a, y);
+  q = fmaf(fmaf(-b, q, a), y, q);
+  return fmaf(fmaf(-b, q, a), y, q);
+}
+// RN(1/b): one Newton step on the hardware's approximation; equal to __frcp_rn for every one of
+// the 2^23 significands, at exponents -60 .. 60 (compared exhaustively on the device).
+__device__ __forceinline__ float rcp_rn(float b) {
+  const float y = rcp_approx(b);
+  return fmaf(fmaf(-b, y, 1.0f), y, y);
+}
+// RN(sqrt(x)) by one Newton step on x * rsqrt(x); equal to __fsqrt_rn for every float from 2^-100
+// to 2^100 (compared exhaustively on the device).  x must not be zero.
+__device__ __forceinline__ float sqrt_rn(float x) {
+  const float y = rsqrt_approx(x);
+  const float g = mul(x, y), h = mul(0.5f, y);
+  return fmaf(fmaf(-g, g, x), h, g);
+}
+
+// (m / bc1) / (sqrt(v / bc2) + eps) for any operands; a call, so that it costs the kernels no registers
+static __device__ __noinline__ float adam_ratio(float m, float v, float bc1, float bc2, float eps) {
+  return fdiv(fdiv(m, bc1), add(fsqrt(fdiv(v, bc2)), eps));
+}
 
 struct AdamOp {
   float lr, beta1, beta2, beta3, one_minus_beta2, eps, bc1, bc2, wd, gscale;
   int mode;
-  __device__ __forceinline__ void operator()(float g, float& p, float& m, float& v) const {
+  float y1, y2;  // RN(1/bc1), RN(1/bc2)
+  int fast;      // bc1, bc2 and eps allow vec() its branch-free form
+  __device__ __forceinline__ void moments(float& g, float p, float& m, float& v) const {
     if (gscale != 1.0f) g = mul(g, gscale);
     if (mode == 0) g = add(g, mul(wd, p));
     m = add(mul(m, beta1), mul(beta3, g));
     v = add(mul(v, beta2), mul(mul(one_minus_beta2, g), g));
-    float denom = add(fsqrt(fdiv(v, bc2)), eps);
-    float update = fdiv(fdiv(m, bc1), denom);
+  }
+  __device__ __forceinline__ void finish(float update, float& p) const {
     if (mode != 0) update = add(update, mul(wd, p));
     p = sub(p, mul(lr, update));
+  }
+  __device__ __forceinline__ void operator()(float g, float& p, float& m, float& v) const {
+    moments(g, p, m, v);
+    finish(adam_ratio(m, v, bc1, bc2, eps), p);
+  }
+  // Four elements at once.  Two exact divisions by per-call constants, one by the denominator and
+  // one square root per element: with the library forms the Adam kernel issued more than HBM
+  // could feed (44,353,792 elements bf16: 215 us).  Here the operands of all four are
+  // tested once and the arithmetic is straight-line code with the same bits.  The test:
+  // m is +0 or 2^-80 .. 2^60 in size, v is +0 or 2^-100 .. 2^40, and the host has seen bc1, bc2 in
+  // 2^-20 .. 1 and eps in 2^-40 .. 1: every quotient is then a normal number or zero, every
+  // remainder exact, and the denominator lies within 2^-40 .. 2^31.
+  __device__ __forceinline__ void vec(const F4& gi, F4& p, F4& m, F4& v) const {
+    bool ok = fast != 0;
+    F4 g = gi;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      moments(g.x[j], p.x[j], m.x[j], v.x[j]);
+      const unsigned mb = __float_as_uint(m.x[j]), vb = __float_as_uint(v.x[j]);
+      ok &= (mb == 0u) | ((mb & 0x7fffffffu) - 0x17800000u < 0x46000000u);  // 2^-80 <= |m| < 2^60
+      ok &= (vb == 0u) | (vb - 0x0d800000u < 0x46000000u);                  // 2^-100 <= v < 2^40
+    }
+    if (__builtin_expect(ok, 1)) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float vh = div_by(v.x[j], bc2, y2);
+        const float denom = add(vh == 0.0f ? 0.0f : sqrt_rn(vh), eps);
+        finish(div_by(div_by(m.x[j], bc1, y1), denom, rcp_rn(denom)), p.x[j]);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) finish(adam_ratio(m.x[j], v.x[j], bc1, bc2, eps), p.x[j]);
+    }
   }
 };
 
@@ -58,17 +140,6 @@ struct AdamOp {
 // Each substitution moves a result by at most about one unit
 // in the last place (1.2e-7 relative); the tests bound the total against the
 // exact restatement at 2e-6 for m and v and far less for p.
-__device__ __forceinline__ float rcp_approx(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float sqrt_approx(float x) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 struct LansStage1 {
   float beta1, beta2, beta3, one_minus_beta2, eps, inv_bc1, inv_bc2, wd, gscale;
   int mode, normalize;
@@ -104,7 +175,59 @@ struct LansStage1 {
   }
 };
 
-// ---- chunk walkers ------------------------------------------------------------
+// ---- the element-wise update of a span --------------------------------------------
+// One block's share: `len` elements (<= kBlockThreads * 4 * UNROLL) of one tensor from element
+// `start`.  Every load of the span is issued before the first use: 256 threads with UNROLL = 2
+// keep 24 to 32 KB in flight per block, and six to eight blocks of them an SM.
+template <int NSTATE, typename GT, typename OT, int UNROLL, typename Op>
+__device__ __forceinline__ void update_span(const TensorDesc& d, int64_t start, int len, const Op& op,
+                                            const Policies& pol) {
+  const GT* g = static_cast<const GT*>(d.g) + start;
+  float* p = d.p + start;
+  float* m = d.m + start;
+  float* v = NSTATE == 2 ? d.v + start : nullptr;
+  OT* out = d.out ? static_cast<OT*>(d.out) + start : nullptr;
+  const int tid = threadIdx.x;
+  int done = 0;
+  if (d.flags & kFlagAligned) {
+    const int len4 = len & ~(kVec - 1);
+    F4 rg[UNROLL], rp[UNROLL], rm[UNROLL], rv[UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int e = u * kPassElems + tid * kVec;
+      if (e < len4) {
+        rg[u] = Elem<GT>::template load4<kStream>(g + e, pol);
+        rp[u] = Elem<float>::template load4<kStream>(p + e, pol);
+        rm[u] = Elem<float>::template load4<kStream>(m + e, pol);
+        if (NSTATE == 2) rv[u] = Elem<float>::template load4<kStream>(v + e, pol);
+        else rv[u] = f4_zero();
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const int e = u * kPassElems + tid * kVec;
+      if (e < len4) {
+        op.vec(rg[u], rp[u], rm[u], rv[u]);
+        Elem<float>::template store4<kDefault>(p + e, rp[u], pol);
+        Elem<float>::template store4<kDefault>(m + e, rm[u], pol);
+        if (NSTATE == 2) Elem<float>::template store4<kDefault>(v + e, rv[u], pol);
+        if (out) Elem<OT>::template store4<kDefault>(out + e, rp[u], pol);
+      }
+    }
+    done = len4;
+  }
+  for (int e = done + tid; e < len; e += kBlockThreads) {
+    float gg = Elem<GT>::to_f32(g[e]);
+    float pp = p[e], mm = m[e], vv = NSTATE == 2 ? v[e] : 0.f;
+    op(gg, pp, mm, vv);
+    p[e] = pp;
+    m[e] = mm;
+    if (NSTATE == 2) v[e] = vv;
+    if (out) out[e] = Elem<OT>::from_f32(pp);
+  }
+}
+
+// What a chunk of the list (fused kernel) covers.
 struct ChunkView {
   const void* g;
   float* p;
@@ -112,7 +235,6 @@ struct ChunkView {
   float* v;
   void* out;
   int len;       // elements in this chunk
-  bool aligned;  // vector path allowed
 };
 
 __device__ __forceinline__ ChunkView chunk_view(const TensorDesc& d, uint32_t chunk, int g_size,
@@ -126,60 +248,7 @@ __device__ __forceinline__ ChunkView chunk_view(const TensorDesc& d, uint32_t ch
   c.m = d.m + start;
   c.v = d.v ? d.v + start : nullptr;
   c.out = d.out ? static_cast<char*>(d.out) + start * out_size : nullptr;
-  c.aligned = (d.flags & kFlagAligned) != 0;
   return c;
-}
-
-// Read-modify-write of p, m (and v when NSTATE == 2) over one chunk.
-template <int NSTATE, typename GT, typename OT, typename Op>
-__device__ __forceinline__ void update_chunk(const ChunkView& c, const Op& op,
-                                             const Policies& pol) {
-  const GT* g = static_cast<const GT*>(c.g);
-  OT* out = static_cast<OT*>(c.out);
-  const int tid = threadIdx.x;
-  int done = 0;
-  if (c.aligned) {
-    const int len4 = c.len & ~(kVec - 1);
-    for (int base = 0; base < len4; base += kUnroll * kPassElems) {
-      F4 rg[kUnroll], rp[kUnroll], rm[kUnroll], rv[kUnroll];
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int e = base + u * kPassElems + tid * kVec;
-        if (e < len4) {
-          rg[u] = Elem<GT>::template load4<kStream>(g + e, pol);
-          rp[u] = Elem<float>::template load4<kStream>(c.p + e, pol);
-          rm[u] = Elem<float>::template load4<kStream>(c.m + e, pol);
-          if (NSTATE == 2) rv[u] = Elem<float>::template load4<kStream>(c.v + e, pol);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kUnroll; ++u) {
-        const int e = base + u * kPassElems + tid * kVec;
-        if (e < len4) {
-#pragma unroll
-          for (int j = 0; j < kVec; ++j) {
-            float vv = NSTATE == 2 ? rv[u].x[j] : 0.f;
-            op(rg[u].x[j], rp[u].x[j], rm[u].x[j], vv);
-            if (NSTATE == 2) rv[u].x[j] = vv;
-          }
-          Elem<float>::template store4<kDefault>(c.p + e, rp[u], pol);
-          Elem<float>::template store4<kDefault>(c.m + e, rm[u], pol);
-          if (NSTATE == 2) Elem<float>::template store4<kDefault>(c.v + e, rv[u], pol);
-          if (out) Elem<OT>::template store4<kDefault>(out + e, rp[u], pol);
-        }
-      }
-    }
-    done = len4;
-  }
-  for (int e = done + tid; e < c.len; e += kBlockThreads) {
-    float gg = Elem<GT>::to_f32(g[e]);
-    float pp = c.p[e], mm = c.m[e], vv = NSTATE == 2 ? c.v[e] : 0.f;
-    op(gg, pp, mm, vv);
-    c.p[e] = pp;
-    c.m[e] = mm;
-    if (NSTATE == 2) c.v[e] = vv;
-    if (out) out[e] = Elem<OT>::from_f32(pp);
-  }
 }
 
 }  // namespace rafb200

@@ -39,6 +39,11 @@ struct Policies {
   }
 };
 
+// Programmatic dependent launch (launch_dependent in common.h): let the next kernel's blocks be
+// placed as soon as every block of this one runs; wait until every earlier kernel is complete.
+__device__ __forceinline__ void grid_dependency_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- raw 16-byte / 8-byte accesses ---------------------------------------
 template <int H>
 __device__ __forceinline__ uint4 ld16(const void* p, const Policies& pol) {

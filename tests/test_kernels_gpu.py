@@ -450,3 +450,28 @@ def test_lans_bounded_wait_reports_instead_of_hanging(rb):
     O.lans([g], [p], [m], [v], 1, **okw)
     assert rel_err(to_numpy(tp), p) < 1e-5 and rel_err(to_numpy(tm), m) < 1e-5
     tl.close()
+
+
+@pytest.mark.parametrize("bias_correction,eps", [(1, 1e-8), (0, 1e-8), (1, 0.0)])
+@pytest.mark.parametrize("n", [3, 2047, 2048, 2049, 6150])
+def test_adam_special_values_bit_exact(rb, n, bias_correction, eps):
+    """Operands on both sides of the ranges in which the kernel's branch-free division and square
+    root are used - zeros of either sign, denormals, tiny, huge, infinite - one kind per element,
+    so that a thread's four elements mix; and spans that end next to a multiple of 2048."""
+    kinds = np.array([0.0, -0.0, 1e-40, 1e-30, 1e-24, 1e-12, 1e-3, -1e-3, 1.0, 1e15, 1e19, 1e25, np.inf], np.float32)
+    rng = np.random.default_rng(n)
+    pick = lambda: kinds[rng.integers(0, kinds.size, n)] * rng.uniform(0.5, 2.0, n).astype(np.float32)
+    with np.errstate(all="ignore"):
+        g, p, m, v = pick(), pick(), pick(), np.abs(pick())
+        v[rng.integers(0, n, max(1, n // 9))] = 0.0
+        tg, tp, tm, tv = (to_torch(x, "float32") for x in (g, p, m, v))
+        tl = rb.TensorList([n], "float32", "float32")
+        tl.bind([tg], [tp], [tm], [tv], None)
+        rb.adam_list_(tl, 3, 1e-4, 0.9, 0.95, eps, bias_correction, 0.1, 1)
+        torch.cuda.synchronize()
+        O.adam(g, p, m, v, 3, 1e-4, 0.9, 0.95, eps, bias_correction, 0.1, 1)
+    for ours, want in ((tp, p), (tm, m), (tv, v)):
+        got = to_numpy(ours)
+        nan = np.isnan(want)  # the sign and payload of a NaN are not defined
+        assert np.array_equal(nan, np.isnan(got)) and bits_equal(got[~nan], want[~nan])
+    tl.close()
