@@ -152,6 +152,17 @@ RAFB200_API int rafb200_tensor_list_set_lans_items(rafb200_tensor_list_t list, c
 RAFB200_API int rafb200_sgd(float* x, const void* dx, int dx_dtype, float* v, int64_t numel,
                             float learning_rate, float mu, float weight_decay, float grad_scale,
                             void* out, int out_dtype, void* stream);
+/* The operator's own form: (x, dx, v) are only read, the results go to x1 and v1 (which may be
+ * x and v; src/op/declare/optimizer.cc:22-44 returns new tensors). */
+RAFB200_API int rafb200_sgd_to(const float* x, const void* dx, int dx_dtype, const float* v, float* x1,
+                               float* v1, int64_t numel, float learning_rate, float mu, void* stream);
+/* k independent in-place updates without a tensor list, up to 512 tensors per launch: what the
+ * eager optimizer (python/raf/optim/sgd.py:41-58) does parameter by parameter.  The tables
+ * travel in the launch; host arrays of k entries, element counts below 2^31, entries may be
+ * empty.  The tensors must not overlap. */
+RAFB200_API int rafb200_sgd_many(int k, float* const* x, const void* const* dx, int dx_dtype,
+                                 float* const* v, const int64_t* numel, float learning_rate, float mu,
+                                 void* stream);
 /* The same update over a bound tensor list in ONE launch (x = p, v = m of the list). */
 RAFB200_API int rafb200_sgd_list(rafb200_tensor_list_t list, float learning_rate, float mu,
                                  float weight_decay, float grad_scale, void* stream);

@@ -50,6 +50,8 @@ SIGNATURES = {
     "rafb200_tensor_list_total_elems": (_i64, [_vp]),
     "rafb200_tensor_list_tune": (_i, [_vp, _i64, _i, _i]),
     "rafb200_sgd": (_i, [_vp, _vp, _i, _vp, _i64, _f, _f, _f, _f, _vp, _i, _vp]),
+    "rafb200_sgd_to": (_i, [_vp, _vp, _i, _vp, _vp, _vp, _i64, _f, _f, _vp]),
+    "rafb200_sgd_many": (_i, [_i, _vp, _vp, _i, _vp, _vp, _f, _f, _vp]),
     "rafb200_sgd_list": (_i, [_vp, _f, _f, _f, _f, _vp]),
     "rafb200_lans_workspace_bytes": (_sz, [_vp]),
     "rafb200_lans": (_i, [_vp, _i, _vp, _f, _f, _f, _f, _i, _f, _i, _i, _i, _f, _vp, _sz, _vp]),
@@ -116,6 +118,23 @@ SIGNATURES = {
 }
 
 _lib = None
+_ops = None
+
+
+def ops():
+    """The native module of the operators (csrc/torch_ops/ops.cc), built first when missing."""
+    global _ops
+    if _ops is None:
+        load()  # libraf_b200.so and torch are in the process before the module links to them
+        if not os.path.exists(os.path.join(HERE, "_ops.so")):
+            from . import build as _build
+
+            _build.build_ops()
+        from . import _ops as mod
+
+        mod.bind(LIB_PATH)
+        _ops = mod
+    return _ops
 
 
 def load() -> C.CDLL:

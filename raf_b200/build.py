@@ -9,6 +9,9 @@ It then compiles the RAF-side glue (``csrc/raf_dialect/b200_ops.cc``) against
 into ``raf_b200/libraf_b200_glue.so``, so that the glue is type-checked and can
 be driven on fake tensors by the tests.  Inside a RAF tree the same file is
 compiled against RAF's own headers instead.
+
+Last comes ``raf_b200/_ops.so`` (``csrc/torch_ops/ops.cc``), the CPython module through which the
+operators reach the library without a detour over ctypes.
 """
 from __future__ import annotations
 
@@ -22,6 +25,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libraf_b200.so")
+OPS_LIB = os.path.join(HERE, "_ops.so")
 GLUE_LIB = os.path.join(HERE, "libraf_b200_glue.so")
 COMPAT = os.path.join(CSRC, "raf_compat")
 
@@ -40,8 +44,8 @@ def _nvcc() -> str:
 def _sources():
     out = []
     for root, _dirs, files in os.walk(CSRC):
-        if "raf_dialect" in root or "raf_compat" in root:
-            continue  # the glue is a library of its own, see build_glue()
+        if "raf_dialect" in root or "raf_compat" in root or "torch_ops" in root:
+            continue  # libraries of their own, see build_glue() and build_ops()
         for f in sorted(files):
             if f.endswith((".cu", ".cc")):
                 out.append(os.path.join(root, f))
@@ -90,7 +94,36 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
             sys.stderr.write(" ".join(link) + "\n" + r.stdout + r.stderr)
             raise RuntimeError("link failed")
     build_glue(nvcc, force or bool(jobs))
+    build_ops(force)
     return LIB
+
+
+def build_ops(force: bool = False) -> str:
+    """ops.cc, a CPython module over torch's C++ API -> _ops.so (host code only)."""
+    src = os.path.join(CSRC, "torch_ops", "ops.cc")
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "raf_b200.h")))
+    if not force and os.path.exists(OPS_LIB) and os.path.getmtime(OPS_LIB) >= newest:
+        return OPS_LIB
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I" + sysconfig.get_paths()["include"], "-I/usr/local/cuda/include"]
+    for d in cpp_extension.include_paths():
+        cmd += ["-isystem", d]
+    cmd += ["-o", OPS_LIB, src]
+    for d in cpp_extension.library_paths():
+        cmd += ["-L" + d, "-Wl,-rpath," + d]
+    cmd += ["-ldl", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu",
+            "-lc10_cuda", "-lc10"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+        raise RuntimeError("building raf_b200._ops failed")
+    return OPS_LIB
 
 
 def build_glue(nvcc: str, force: bool = False) -> str:

@@ -156,6 +156,73 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE, GT>)
   update_span<NSTATE, GT, OT, kSpanUnroll>(d, start, left < kSpanElems ? (int)left : kSpanElems, op, pol);
 }
 
+// SGD from (x, dx, v) to (x1, v1): the operator's own form, which leaves its inputs alone.
+// One pass over 20 bytes an element instead of two clones and an in-place update (36 bytes,
+// three launches); in place when x1 == x and v1 == v.
+template <typename GT>
+__global__ void __launch_bounds__(kBlockThreads)
+    sgd_to_kernel(const GT* g, const float* x, const float* v, float* x1, float* v1, int64_t n, bool aligned,
+                  SgdOp op) {
+  Policies pol;
+  pol.init();
+  grid_dependency_trigger();
+  grid_dependency_wait();
+  const int64_t start = (int64_t)blockIdx.x * kPassElems + threadIdx.x * kVec;
+  if (aligned && start + kVec <= n) {
+    const F4 gg = Elem<GT>::template load4<kStream>(g + start, pol);
+    F4 pp = Elem<float>::template load4<kStream>(x + start, pol);
+    F4 mm = Elem<float>::template load4<kStream>(v + start, pol), unused = f4_zero();
+    op.vec(gg, pp, mm, unused);
+    Elem<float>::template store4<kDefault>(x1 + start, pp, pol);
+    Elem<float>::template store4<kDefault>(v1 + start, mm, pol);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < kVec; ++j) {
+    const int64_t e = start + j;
+    if (e >= n) return;
+    float pp = x[e], mm = v[e], unused = 0.f;
+    op(Elem<GT>::to_f32(g[e]), pp, mm, unused);
+    x1[e] = pp;
+    v1[e] = mm;
+  }
+}
+
+// Tensors described by value, for callers without a tensor list: what an eager loop updates in
+// one launch.  `end` counts spans: block b works on the tensor with end[i - 1] <= b < end[i].
+template <int CAP>
+struct Rows {
+  const void* g[CAP];
+  float* p[CAP];
+  float* m[CAP];
+  uint32_t end[CAP];
+  uint32_t numel[CAP];  // below 2^31; the top bit set = vector accesses allowed
+};
+constexpr int kMaxRows = 512;  // 16 KB of the 32 KB a launch's parameters may take
+
+template <typename GT, int CAP>
+__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<1, GT>)
+    sgd_rows_kernel(const __grid_constant__ Rows<CAP> rows, int k, SgdOp op) {
+  Policies pol;
+  pol.init();
+  grid_dependency_trigger();
+  int lo = 0, hi = k - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (blockIdx.x < rows.end[mid]) hi = mid;
+    else lo = mid + 1;
+  }
+  TensorDesc d{};
+  d.g = rows.g[lo];
+  d.p = rows.p[lo];
+  d.m = rows.m[lo];
+  d.flags = (rows.numel[lo] >> 31) ? kFlagAligned : 0u;
+  const int64_t n = rows.numel[lo] & 0x7fffffffu;
+  const int64_t start = (int64_t)(blockIdx.x - (lo ? rows.end[lo - 1] : 0u)) * kSpanElems;
+  grid_dependency_wait();
+  update_span<1, GT, float, kSpanUnroll>(d, start, n - start < kSpanElems ? (int)(n - start) : kSpanElems, op, pol);
+}
+
 static int grid_for(uint32_t nitems, int device) {
   static int sm_count[64] = {0};
   if (device < 0 || device >= 64) device = 0;
@@ -237,6 +304,42 @@ bool pointers_aligned(const void* g, int g_dtype, const void* p, const void* m, 
   if (v) a = a && ok(v, 16);
   if (out) a = a && ok(out, out_dtype == RAFB200_F32 ? 16 : 8);
   return a;
+}
+
+template <typename GT>
+static int launch_sgd_to(const float* x, const void* dx, const float* v, float* x1, float* v1, int64_t n, bool aligned,
+                         const SgdOp& op, cudaStream_t s) {
+  const unsigned grid = (unsigned)((n + kPassElems - 1) / kPassElems);
+  RAFB200_CUDA(launch_dependent(sgd_to_kernel<GT>, grid, kBlockThreads, 0, s, static_cast<const GT*>(dx), x, v, x1, v1, n,
+                                aligned, op));
+  return RAFB200_OK;
+}
+
+// One launch over k >= 1 tensors, none empty, at most CAP of them.
+template <typename GT, int CAP>
+static int launch_sgd_rows(int k, float* const* x, const void* const* dx, int dx_dtype, float* const* v,
+                           const int64_t* numel, const SgdOp& op, cudaStream_t s) {
+  Rows<CAP> rows;
+  uint64_t end = 0;
+  for (int i = 0; i < k; ++i) {
+    rows.g[i] = dx[i];
+    rows.p[i] = x[i];
+    rows.m[i] = v[i];
+    end += (uint64_t)((numel[i] + kSpanElems - 1) / kSpanElems);
+    rows.end[i] = (uint32_t)end;
+    rows.numel[i] = (uint32_t)numel[i] |
+                    (pointers_aligned(dx[i], dx_dtype, x[i], v[i], nullptr, nullptr, RAFB200_F32) ? 0x80000000u : 0u);
+  }
+  RAFB200_CUDA(launch_dependent(sgd_rows_kernel<GT, CAP>, (unsigned)end, kBlockThreads, 0, s, rows, k, op));
+  return RAFB200_OK;
+}
+
+// The parameter block of a launch is copied whole: the smaller table where it is enough.
+template <typename GT>
+static int launch_sgd_many(int k, float* const* x, const void* const* dx, int dx_dtype, float* const* v,
+                           const int64_t* numel, const SgdOp& op, cudaStream_t s) {
+  if (k <= 64) return launch_sgd_rows<GT, 64>(k, x, dx, dx_dtype, v, numel, op, s);
+  return launch_sgd_rows<GT, kMaxRows>(k, x, dx, dx_dtype, v, numel, op, s);
 }
 
 // Bias corrections exactly as the reference's host code computes them
@@ -417,6 +520,52 @@ int rafb200_sgd(float* x, const void* dx, int dx_dtype, float* v, int64_t numel,
     case RAFB200_F16: return launch_flat_sgd_out<__half>(d, out_dtype, op, s);
     default: return launch_flat_sgd_out<__nv_bfloat16>(d, out_dtype, op, s);
   }
+}
+
+int rafb200_sgd_to(const float* x, const void* dx, int dx_dtype, const float* v, float* x1, float* v1, int64_t numel,
+                   float learning_rate, float mu, void* stream) {
+  RAFB200_REQUIRE(numel >= 0, "rafb200_sgd_to: negative numel");
+  RAFB200_REQUIRE(dtype_valid(dx_dtype), "rafb200_sgd_to: bad dtype");
+  if (numel == 0) return RAFB200_OK;
+  RAFB200_REQUIRE(x && dx && v && x1 && v1, "rafb200_sgd_to: NULL argument");
+  RAFB200_REQUIRE((numel + kPassElems - 1) / kPassElems < (int64_t)1 << 31, "rafb200_sgd_to: tensor too large");
+  const bool aligned = pointers_aligned(dx, dx_dtype, x, v, x1, v1, RAFB200_F32);
+  const SgdOp op{learning_rate, mu, 0.0f, 1.0f};
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (dx_dtype) {
+    case RAFB200_F32: return launch_sgd_to<float>(x, dx, v, x1, v1, numel, aligned, op, s);
+    case RAFB200_F16: return launch_sgd_to<__half>(x, dx, v, x1, v1, numel, aligned, op, s);
+    default: return launch_sgd_to<__nv_bfloat16>(x, dx, v, x1, v1, numel, aligned, op, s);
+  }
+}
+
+int rafb200_sgd_many(int k, float* const* x, const void* const* dx, int dx_dtype, float* const* v,
+                     const int64_t* numel, float learning_rate, float mu, void* stream) {
+  RAFB200_REQUIRE(k >= 0 && (k == 0 || (x && dx && v && numel)), "rafb200_sgd_many: bad arguments");
+  RAFB200_REQUIRE(dtype_valid(dx_dtype), "rafb200_sgd_many: bad dtype");
+  for (int i = 0; i < k; ++i) {
+    RAFB200_REQUIRE(numel[i] >= 0 && numel[i] < (1ll << 31), "rafb200_sgd_many: numel[%d] must be in [0, 2^31)", i);
+    RAFB200_REQUIRE(numel[i] == 0 || (x[i] && dx[i] && v[i]), "rafb200_sgd_many: NULL pointer for tensor %d", i);
+  }
+  const SgdOp op{learning_rate, mu, 0.0f, 1.0f};
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  for (int i = 0; i < k;) {
+    if (numel[i] == 0) {
+      ++i;
+      continue;
+    }
+    int n = 1;  // a run of tensors with elements
+    while (i + n < k && n < kMaxRows && numel[i + n] > 0) ++n;
+    int rc;
+    switch (dx_dtype) {
+      case RAFB200_F32: rc = launch_sgd_many<float>(n, x + i, dx + i, dx_dtype, v + i, numel + i, op, s); break;
+      case RAFB200_F16: rc = launch_sgd_many<__half>(n, x + i, dx + i, dx_dtype, v + i, numel + i, op, s); break;
+      default: rc = launch_sgd_many<__nv_bfloat16>(n, x + i, dx + i, dx_dtype, v + i, numel + i, op, s); break;
+    }
+    if (rc != RAFB200_OK) return rc;
+    i += n;
+  }
+  return RAFB200_OK;
 }
 
 int rafb200_sgd_list(rafb200_tensor_list_t list, float learning_rate, float mu,

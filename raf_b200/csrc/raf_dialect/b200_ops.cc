@@ -127,12 +127,9 @@ class SgdB200 : public OpEnv {
     DLTensor* v1 = ir::Downcast<TensorValue>(out->fields[0]);
     DLTensor* x1 = ir::Downcast<TensorValue>(out->fields[1]);
     const int64_t n = Numel(x);
-    auto s = static_cast<cudaStream_t>(stream_);
-    if (v1->data != v->data) CUDA_CALL(cudaMemcpyAsync(v1->data, v->data, 4 * n, cudaMemcpyDeviceToDevice, s));
-    if (x1->data != x->data) CUDA_CALL(cudaMemcpyAsync(x1->data, x->data, 4 * n, cudaMemcpyDeviceToDevice, s));
-    Check(rafb200_sgd(static_cast<float*>(x1->data), dx->data, DTypeOf(dx, &error_msgs),
-                      static_cast<float*>(v1->data), n, lr_, mu_, /*weight_decay=*/0.f,
-                      /*grad_scale=*/1.f, /*out=*/nullptr, RAFB200_F32, stream_));
+    Check(rafb200_sgd_to(static_cast<const float*>(x->data), dx->data, DTypeOf(dx, &error_msgs),
+                         static_cast<const float*>(v->data), static_cast<float*>(x1->data),
+                         static_cast<float*>(v1->data), n, lr_, mu_, stream_));
   }
   static OpEnv* make(const CallValues& cv) { return new SgdB200(cv); }
 };

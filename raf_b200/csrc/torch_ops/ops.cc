@@ -1,0 +1,185 @@
+// raf_b200._ops: the host side of the operators that are called once per step or per tensor, on
+// torch tensors.  Through ctypes and Python a call cost 10 us before it reached the C ABI
+// (argument conversion, per-tensor checks, stream lookup), several times what a small launch takes.
+//
+// Every function takes the fast way only: when an argument is anything but what the operator
+// expects (another type or device, not contiguous, part of an autograd graph), it returns None and has
+// done nothing - the Python caller then runs its own checks, which raise.  A failed C ABI call
+// returns its status as an int.
+#include <Python.h>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <dlfcn.h>
+
+#include <algorithm>
+#include <vector>
+
+#include "../../../include/raf_b200.h"
+
+namespace {
+
+// The C ABI of the library that the package has loaded (it need not be the one beside this
+// module): bind(path) looks the functions up.
+struct {
+  decltype(&rafb200_sgd_to) sgd_to;
+  decltype(&rafb200_sgd_many) sgd_many;
+} abi;
+
+PyObject* bind(PyObject*, PyObject* path) {
+  const char* p = PyUnicode_AsUTF8(path);
+  if (!p) return nullptr;
+  void* lib = dlopen(p, RTLD_NOW | RTLD_NOLOAD);
+  if (!lib) return PyErr_Format(PyExc_ImportError, "%s is not loaded", p);
+  auto find = [&](auto& fn, const char* name) {
+    fn = reinterpret_cast<std::remove_reference_t<decltype(fn)>>(dlsym(lib, name));
+    if (!fn) PyErr_Format(PyExc_ImportError, "%s has no %s", p, name);
+    return fn != nullptr;
+  };
+  if (!find(abi.sgd_to, "rafb200_sgd_to") || !find(abi.sgd_many, "rafb200_sgd_many")) return nullptr;
+  Py_RETURN_NONE;
+}
+
+int code_of(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return RAFB200_F32;
+    case at::kHalf: return RAFB200_F16;
+    case at::kBFloat16: return RAFB200_BF16;
+    default: return -1;
+  }
+}
+
+// A dense CUDA tensor on the current device, or nullptr.
+const at::Tensor* plain(PyObject* o, c10::DeviceIndex device) {
+  if (!THPVariable_Check(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  if (!t.defined() || t.layout() != at::kStrided || !t.is_cuda() || t.device().index() != device || !t.is_contiguous())
+    return nullptr;
+  return &t;
+}
+
+// The same outside any autograd graph.
+const at::Tensor* data_only(PyObject* o, c10::DeviceIndex device) {
+  const at::Tensor* t = plain(o, device);
+  return t && !t->requires_grad() ? t : nullptr;
+}
+
+void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
+
+PyObject* nothing() { Py_RETURN_NONE; }
+
+// sgd(x, dx, v, learning_rate, mu) -> (v1, x1)
+PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 5) return nothing();
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  const at::Tensor *x = data_only(a[0], dev), *dx = data_only(a[1], dev), *v = data_only(a[2], dev);
+  if (!x || !dx || !v) return nothing();
+  const int code = code_of(dx->scalar_type());
+  const double lr = PyFloat_AsDouble(a[3]), mu = PyFloat_AsDouble(a[4]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return nothing();
+  }
+  if (x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat || code < 0 || x->sizes() != dx->sizes() ||
+      x->sizes() != v->sizes())
+    return nothing();
+  at::Tensor x1 = at::detail::empty_cuda(x->sizes(), at::kFloat, x->device(), c10::nullopt);
+  at::Tensor v1 = at::detail::empty_cuda(x->sizes(), at::kFloat, x->device(), c10::nullopt);
+  const int rc = abi.sgd_to(x->const_data_ptr<float>(), dx->const_data_ptr(), code, v->const_data_ptr<float>(),
+                                x1.mutable_data_ptr<float>(), v1.mutable_data_ptr<float>(), x->numel(), (float)lr, (float)mu,
+                                current_stream(dev));
+  if (rc != RAFB200_OK) return PyLong_FromLong(rc);
+  PyObject* out = PyTuple_New(2);
+  if (!out) return nullptr;
+  PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(v1)));
+  PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(std::move(x1)));
+  return out;
+}
+
+// Do the byte ranges overlap anywhere, ranges that are only read among themselves excepted?
+struct Range {
+  uintptr_t lo, hi;
+  bool written;
+};
+bool overlap(std::vector<Range>& r) {
+  std::sort(r.begin(), r.end(), [](const Range& p, const Range& q) { return p.lo < q.lo; });
+  uintptr_t any = 0, written = 0;  // the furthest ends so far
+  for (const Range& x : r) {
+    if (x.lo == x.hi) continue;
+    if (x.lo < (x.written ? any : written)) return true;
+    any = std::max(any, x.hi);
+    if (x.written) written = std::max(written, x.hi);
+  }
+  return false;
+}
+
+// sgd_step([(x, v), ...], learning_rate, mu) -> True: every x with a gradient updated in place, one
+// launch for all of them.
+PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 3 || !PyList_CheckExact(a[0])) return nothing();
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  const double lr = PyFloat_AsDouble(a[1]), mu = PyFloat_AsDouble(a[2]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return nothing();
+  }
+  const Py_ssize_t k = PyList_GET_SIZE(a[0]);
+  std::vector<float*> xs, vs;
+  std::vector<const void*> gs;
+  std::vector<int64_t> numel;
+  std::vector<Range> ranges;
+  xs.reserve(k);
+  vs.reserve(k);
+  gs.reserve(k);
+  numel.reserve(k);
+  ranges.reserve(3 * k);
+  int code = -1;
+  for (Py_ssize_t i = 0; i < k; ++i) {
+    PyObject* pair = PyList_GET_ITEM(a[0], i);
+    if (!PyTuple_CheckExact(pair) || PyTuple_GET_SIZE(pair) != 2) return nothing();
+    const at::Tensor *x = plain(PyTuple_GET_ITEM(pair, 0), dev), *v = plain(PyTuple_GET_ITEM(pair, 1), dev);
+    if (!x || !v) return nothing();
+    const at::Tensor& g = x->grad();
+    if (!g.defined()) continue;
+    const int c = code_of(g.scalar_type());
+    if (g.layout() != at::kStrided || !g.is_cuda() || g.device() != x->device() || !g.is_contiguous() || c < 0 ||
+        (code >= 0 && c != code) || x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat ||
+        g.numel() != x->numel() || v->numel() != x->numel() || x->numel() >= (int64_t(1) << 31))
+      return nothing();
+    code = c;
+    const int64_t ne = x->numel();
+    float* xp = static_cast<float*>(x->data_ptr());
+    float* vp = static_cast<float*>(v->data_ptr());
+    const void* gp = g.const_data_ptr();
+    xs.push_back(xp);
+    vs.push_back(vp);
+    gs.push_back(gp);
+    numel.push_back(ne);
+    const uintptr_t xb = reinterpret_cast<uintptr_t>(xp), vb = reinterpret_cast<uintptr_t>(vp),
+                    gb = reinterpret_cast<uintptr_t>(gp);
+    ranges.push_back({xb, xb + ne * 4, true});
+    ranges.push_back({vb, vb + ne * 4, true});
+    ranges.push_back({gb, gb + ne * g.element_size(), false});
+  }
+  if (overlap(ranges)) return nothing();  // tied parameters: one after the other, as the loop does
+  if (!xs.empty()) {
+    const int rc = abi.sgd_many((int)xs.size(), xs.data(), gs.data(), code, vs.data(), numel.data(), (float)lr,
+                                    (float)mu, current_stream(dev));
+    if (rc != RAFB200_OK) return PyLong_FromLong(rc);
+  }
+  Py_RETURN_TRUE;
+}
+
+PyMethodDef kMethods[] = {
+    {"bind", bind, METH_O, "use the C ABI of the loaded library at this path"},
+    {"sgd", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd)), METH_FASTCALL, "raf.op.sgd"},
+    {"sgd_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd_step)), METH_FASTCALL, "eager SGD, all parameters"},
+    {nullptr, nullptr, 0, nullptr}};
+
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ops", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__ops() { return PyModule_Create(&kModule); }

@@ -133,6 +133,11 @@ class TensorList:
 # --------------------------------------------------------------------------- optimizers
 def sgd(x, dx, v, learning_rate, mu):
     """raf.op.sgd: returns (v1, x1) as NEW tensors (src/op/declare/optimizer.cc:22-44)."""
+    r = _lib.ops().sgd(x, dx, v, learning_rate, mu)
+    if r.__class__ is tuple:
+        return r
+    if r is not None:
+        check(r)
     _check_cuda(x, dx, v)
     if x.shape != dx.shape or x.shape != v.shape:
         raise ValueError("sgd: x, dx and v must have the same shape")

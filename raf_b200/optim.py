@@ -15,6 +15,7 @@ from typing import Dict, Iterable, List, Optional, Sequence
 
 import torch
 
+from . import _lib
 from . import distributed as dist
 from . import op
 from .zero import Plan, ZeroStep, make_hyper
@@ -40,7 +41,13 @@ class SGD:
         return {f"sgd.{i}.v": v for i, (_, v) in enumerate(self.params)}
 
     def step(self):
-        """Update the parameters with gradients."""
+        """Update the parameters with gradients: one launch where they are separate fp32 tensors
+        on one device, else one after the other."""
+        done = _lib.ops().sgd_step(self.params, self._lr, self._momentum)
+        if done is True:
+            return
+        if done is not None:
+            _lib.check(done)
         for x0, v0 in self.params:
             if x0.grad is None:
                 continue

@@ -475,3 +475,55 @@ def test_adam_special_values_bit_exact(rb, n, bias_correction, eps):
         nan = np.isnan(want)  # the sign and payload of a NaN are not defined
         assert np.array_equal(nan, np.isnan(got)) and bits_equal(got[~nan], want[~nan])
     tl.close()
+
+
+@pytest.mark.parametrize("g_dtype", G_DTYPES)
+@pytest.mark.parametrize("n", [1, 3, 1023, 1024, 1025, 4097])
+def test_sgd_op_out_of_place_bit_exact(rb, n, g_dtype):
+    """The operator's one-pass form around the edges of a block's 1024 elements, aligned and not."""
+    rng = np.random.default_rng(n)
+    p, v, _ = _params(rng, n)
+    v = (rng.standard_normal(n) * 1e-3).astype(np.float32)
+    g = make_grad(rng, n, g_dtype)
+    for off in (0, 1):
+        tp, tv = (torch.zeros(n + 1, device="cuda")[off:off + n] for _ in range(2))
+        tp.copy_(torch.from_numpy(p))
+        tv.copy_(torch.from_numpy(v))
+        v1, x1 = rb.sgd(tp, to_torch(g, g_dtype), tv, 0.1, 0.9)
+        wp, wv = p.copy(), v.copy()
+        O.sgd(wp, g, wv, 0.1, 0.9)
+        assert bits_equal(to_numpy(x1), wp) and bits_equal(to_numpy(v1), wv)
+        assert bits_equal(to_numpy(tp), p) and bits_equal(to_numpy(tv), v)
+
+
+@pytest.mark.parametrize("count", [1, 64, 65, 600])
+def test_sgd_eager_step_one_launch_bit_exact(rb, count):
+    """optim.SGD around the table sizes of the one-launch step: empty tensors, parameters without a
+    gradient, unaligned views, and tied parameters (updated twice, one after the other)."""
+    from raf_b200.optim import SGD
+
+    rng = np.random.default_rng(count)
+    sizes = [int(s) for s in rng.choice([0, 1, 5, 2047, 2048, 2049, 4099], count)]
+    ps = [(rng.standard_normal(n) * 0.02).astype(np.float32) for n in sizes]
+    xs = []
+    for i, p in enumerate(ps):
+        x = torch.zeros(p.size + 1, device="cuda")[i % 2:i % 2 + p.size]
+        x.copy_(torch.from_numpy(p))
+        xs.append(x)
+    tied = count == 65
+    opt = SGD(xs + ([xs[3]] if tied else []), 0.1, 0.9)
+    vs = [np.zeros(n, np.float32) for n in sizes]
+    v_tied = np.zeros(sizes[3] if tied else 0, np.float32)
+    for step in range(2):
+        gs = [make_grad(rng, n, "float32") for n in sizes]
+        for i, (x, g) in enumerate(zip(xs, gs)):
+            x.grad = None if i % 7 == 6 else to_torch(g, "float32")
+            if i % 7 != 6:
+                O.sgd(ps[i], g, vs[i], 0.1, 0.9)
+        if tied:
+            O.sgd(ps[3], gs[3], v_tied, 0.1, 0.9)
+        opt.step()
+    for i, (x, _) in enumerate(opt.params[:count]):
+        assert bits_equal(to_numpy(x), ps[i]) and bits_equal(to_numpy(opt.state()[f"sgd.{i}.v"]), vs[i]), i
+    if tied:
+        assert bits_equal(to_numpy(opt.state()[f"sgd.{count}.v"]), v_tied)
