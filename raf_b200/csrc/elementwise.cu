@@ -408,86 +408,188 @@ static int cast_impl(const void* src, int src_dtype, void* dst, int dst_dtype, i
   }
 }
 
-// ---- batched byte movers (group_cast, fuse_tensor, defuse_tensor) -----------
-constexpr int kBatch = 96;  // tensors per launch: 96 * 24 B of pointers/sizes fit the 4 KB parameter space
-struct CopyBatch {
-  const void* src[kBatch];
-  void* dst[kBatch];
-  int64_t numel[kBatch];
+// ---- batched movers (group_cast, fuse_tensor, defuse_tensor) ------------------------
+// Bound: HBM, and for a bucket of small tensors the launch.  The tensors travel in the launch
+// parameters; one block per span of one tensor, found by bisection over the running span counts
+// (a grid as wide as the largest tensor for every tensor left most blocks of a ragged list empty).
+template <int CAP>
+struct CopyRows {
+  const void* src[CAP];
+  void* dst[CAP];
+  int64_t count[CAP];  // elements of a cast, bytes of a copy
+  uint32_t end[CAP];   // spans of tensors 0 .. i
 };
+constexpr int kFewRows = 64;  // launches with no more tensors pass the smaller table
 
-template <typename ST, typename DT>
-__global__ void __launch_bounds__(kBlockThreads) group_cast_kernel(CopyBatch b) {
-  const int t = blockIdx.y;
-  const ST* src = static_cast<const ST*>(b.src[t]);
-  DT* dst = static_cast<DT*>(b.dst[t]);
-  const int64_t n = b.numel[t];
+template <int CAP>
+__device__ __forceinline__ int row_of(const CopyRows<CAP>& r, int k) {
+  int lo = 0, hi = k - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (blockIdx.x < r.end[mid]) hi = mid;
+    else lo = mid + 1;
+  }
+  return lo;
+}
+
+constexpr int kCastUnroll = 4;
+constexpr int kCastSpan = kPassElems * kCastUnroll;  // elements per block
+template <typename ST, typename DT, int CAP>
+__global__ void __launch_bounds__(kBlockThreads) group_cast_kernel(const __grid_constant__ CopyRows<CAP> rows, int k) {
+  Policies pol;
+  pol.init();
+  grid_dependency_trigger();
+  const int t = row_of(rows, k);
+  const int64_t start = (int64_t)(blockIdx.x - (t ? rows.end[t - 1] : 0u)) * kCastSpan;
+  const ST* src = static_cast<const ST*>(rows.src[t]) + start;
+  DT* dst = static_cast<DT*>(rows.dst[t]) + start;
+  const int64_t left = rows.count[t] - start;
+  const int len = left < kCastSpan ? (int)left : kCastSpan;
   const bool aligned = (reinterpret_cast<uintptr_t>(src) % (sizeof(ST) * 4) == 0) &&
                        (reinterpret_cast<uintptr_t>(dst) % (sizeof(DT) * 4) == 0);
-  Policies pol;
-  pol.init();
-  const int64_t n4 = aligned ? (n & ~(int64_t)3) : 0;
-  for (int64_t e = ((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) * 4; e < n4;
-       e += (int64_t)gridDim.x * kBlockThreads * 4) {
-    F4 v = Elem<ST>::template load4<kStream>(src + e, pol);
-    Elem<DT>::template store4<kDefault>(dst + e, v, pol);
+  const int len4 = aligned ? (len & ~3) : 0;
+  grid_dependency_wait();
+  F4 v[kCastUnroll];
+#pragma unroll
+  for (int u = 0; u < kCastUnroll; ++u) {
+    const int e = u * kPassElems + threadIdx.x * kVec;
+    if (e < len4) v[u] = Elem<ST>::template load4<kStream>(src + e, pol);
   }
-  for (int64_t e = n4 + (int64_t)blockIdx.x * kBlockThreads + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * kBlockThreads)
-    dst[e] = Elem<DT>::from_f32(Elem<ST>::to_f32(src[e]));
+#pragma unroll
+  for (int u = 0; u < kCastUnroll; ++u) {
+    const int e = u * kPassElems + threadIdx.x * kVec;
+    if (e < len4) Elem<DT>::template store4<kDefault>(dst + e, v[u], pol);
+  }
+  for (int e = len4 + threadIdx.x; e < len; e += kBlockThreads) dst[e] = Elem<DT>::from_f32(Elem<ST>::to_f32(src[e]));
 }
 
-// Plain byte copy of each (src, dst, nbytes) triple; 16-byte accesses when both ends allow.
-__global__ void __launch_bounds__(kBlockThreads) group_copy_kernel(CopyBatch b) {
-  const int t = blockIdx.y;
-  const char* src = static_cast<const char*>(b.src[t]);
-  char* dst = static_cast<char*>(b.dst[t]);
-  const int64_t n = b.numel[t];  // bytes
-  const bool aligned = (reinterpret_cast<uintptr_t>(src) % 16 == 0) &&
-                       (reinterpret_cast<uintptr_t>(dst) % 16 == 0);
+// 16 bytes that start `sh` bytes (1 .. 15) into the two aligned words a, b.
+__device__ __forceinline__ uint4 shifted(uint4 a, uint4 b, int sh) {
+  const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const int r = (sh & 3) * 8;
+  uint4 o;
+#define RAFB200_SHIFTED(Q)                       \
+  case Q:                                        \
+    o.x = __funnelshift_r(w[Q], w[Q + 1], r);     \
+    o.y = __funnelshift_r(w[Q + 1], w[Q + 2], r); \
+    o.z = __funnelshift_r(w[Q + 2], w[Q + 3], r); \
+    o.w = __funnelshift_r(w[Q + 3], w[Q < 3 ? Q + 4 : 7], r); \
+    break;
+  switch (sh >> 2) {
+    RAFB200_SHIFTED(0)
+    RAFB200_SHIFTED(1)
+    RAFB200_SHIFTED(2)
+    default:
+      RAFB200_SHIFTED(3)
+  }
+#undef RAFB200_SHIFTED
+  return o;
+}
+
+// Byte copies.  Where source and destination lie differently to 16 bytes (a tensor of odd size
+// in front of this one in the flat buffer), the destination is still written in aligned 16-byte
+// words: each is cut out of the two aligned source words it spans.  Words of which a source half
+// would lie outside the tensor, and the bytes before the first and after the last word, go
+// byte by byte.  48 ragged fp32 tensors, 13.5 MB, packed and unpacked: see rafb200_fuse_tensor.
+constexpr int kCopyUnroll = 2;
+constexpr int kCopySpan = kBlockThreads * 16 * kCopyUnroll;  // bytes per block
+template <int CAP>
+__global__ void __launch_bounds__(kBlockThreads) group_copy_kernel(const __grid_constant__ CopyRows<CAP> rows, int k) {
   Policies pol;
   pol.init();
-  const int64_t n16 = aligned ? (n & ~(int64_t)15) : 0;
-  for (int64_t e = ((int64_t)blockIdx.x * kBlockThreads + threadIdx.x) * 16; e < n16;
-       e += (int64_t)gridDim.x * kBlockThreads * 16)
-    st16<kDefault>(dst + e, ld16<kStream>(src + e, pol), pol);
-  for (int64_t e = n16 + (int64_t)blockIdx.x * kBlockThreads + threadIdx.x; e < n;
-       e += (int64_t)gridDim.x * kBlockThreads)
-    dst[e] = src[e];
-}
-
-template <typename Launch>
-static int for_each_batch(int k, const void* const* src, void* const* dst, const int64_t* numel,
-                          int64_t scale, int work_per_thread, Launch launch) {
-  for (int t0 = 0; t0 < k; t0 += kBatch) {
-    CopyBatch b;
-    const int nb = (k - t0 < kBatch) ? k - t0 : kBatch;
-    int64_t maxn = 0;
-    for (int i = 0; i < nb; ++i) {
-      b.src[i] = src[t0 + i];
-      b.dst[i] = dst[t0 + i];
-      b.numel[i] = numel[t0 + i] * scale;
-      if (b.numel[i] > maxn) maxn = b.numel[i];
+  grid_dependency_trigger();
+  const int t = row_of(rows, k);
+  const int64_t start = (int64_t)(blockIdx.x - (t ? rows.end[t - 1] : 0u)) * kCopySpan;
+  const char* const row = static_cast<const char*>(rows.src[t]);
+  const char* const row_end = row + rows.count[t];
+  const int64_t left = rows.count[t] - start;
+  const int len = left < kCopySpan ? (int)left : kCopySpan;
+  const char* src = row + start;
+  char* dst = static_cast<char*>(rows.dst[t]) + start;
+  int head = (int)(-reinterpret_cast<intptr_t>(dst) & 15);
+  if (head > len) head = len;
+  const int nv = (len - head) >> 4;
+  const int sh = (int)(reinterpret_cast<uintptr_t>(src + head) & 15);
+  grid_dependency_wait();
+  uint4 v[kCopyUnroll];
+  bool whole[kCopyUnroll];
+#pragma unroll
+  for (int u = 0; u < kCopyUnroll; ++u) {
+    const int i = threadIdx.x + u * kBlockThreads;
+    const char* s = src + head + (size_t)i * 16 - sh;
+    whole[u] = i < nv && (sh == 0 || (s >= row && s + 32 <= row_end));
+    if (whole[u]) v[u] = sh == 0 ? ld16<kStream>(s, pol) : shifted(ld16<kDefault>(s, pol), ld16<kDefault>(s + 16, pol), sh);
+  }
+#pragma unroll
+  for (int u = 0; u < kCopyUnroll; ++u) {
+    const int i = threadIdx.x + u * kBlockThreads;
+    if (whole[u]) {
+      st16<kDefault>(dst + head + (size_t)i * 16, v[u], pol);
+    } else if (i < nv) {
+      for (int j = 0; j < 16; ++j) dst[head + i * 16 + j] = src[head + i * 16 + j];
     }
-    if (maxn == 0) continue;
-    const int64_t per_block = (int64_t)kBlockThreads * work_per_thread;
-    int64_t gx = (maxn + per_block - 1) / per_block;
-    if (gx > 148 * 4) gx = 148 * 4;
-    int rc = launch(b, dim3((unsigned)gx, (unsigned)nb));
-    if (rc != RAFB200_OK) return rc;
   }
-  return RAFB200_OK;
+  if ((int)threadIdx.x < head) dst[threadIdx.x] = src[threadIdx.x];
+  const int tail = head + nv * 16 + threadIdx.x;
+  if (tail < len) dst[tail] = src[tail];
+}
+
+// Calls `launch(rows, k, spans)` for the tensors in groups that fit a table; empty ones are left out.
+template <int CAP, typename Launch>
+static int for_each_group(int k, const void* const* src, void* const* dst, const int64_t* numel, int64_t scale, int span,
+                          Launch launch) {
+  CopyRows<CAP> rows;
+  int n = 0;
+  uint64_t spans = 0;
+  for (int i = 0; i < k; ++i) {
+    const int64_t count = numel[i] * scale;
+    const uint64_t mine = (uint64_t)((count + span - 1) / span);
+    if (n == CAP || (n > 0 && spans + mine >= (1ull << 31))) {
+      if (int rc = launch(rows, n, (unsigned)spans)) return rc;
+      n = 0;
+      spans = 0;
+    }
+    if (count == 0) continue;
+    spans += mine;
+    rows.src[n] = src[i];
+    rows.dst[n] = dst[i];
+    rows.count[n] = count;
+    rows.end[n++] = (uint32_t)spans;
+  }
+  return n ? launch(rows, n, (unsigned)spans) : (int)RAFB200_OK;
+}
+
+template <typename ST, typename DT, int CAP>
+static int group_cast_rows(int k, const void* const* src, void* const* dst, const int64_t* numel, cudaStream_t s) {
+  return for_each_group<CAP>(k, src, dst, numel, 1, kCastSpan, [&](const CopyRows<CAP>& r, int n, unsigned spans) {
+    RAFB200_CUDA(launch_dependent(group_cast_kernel<ST, DT, CAP>, spans, kBlockThreads, 0, s, r, n));
+    return (int)RAFB200_OK;
+  });
+}
+
+template <typename ST, typename DT>
+static int group_cast_any(int k, const void* const* src, void* const* dst, const int64_t* numel, cudaStream_t s) {
+  return k <= kFewRows ? group_cast_rows<ST, DT, kFewRows>(k, src, dst, numel, s)
+                       : group_cast_rows<ST, DT, kMaxRows>(k, src, dst, numel, s);
 }
 
 template <typename ST>
-static int group_cast_dst(const CopyBatch& b, dim3 grid, int dst_dtype, cudaStream_t s) {
+static int group_cast_dst(int k, const void* const* src, void* const* dst, int dst_dtype, const int64_t* numel,
+                          cudaStream_t s) {
   switch (dst_dtype) {
-    case RAFB200_F32: group_cast_kernel<ST, float><<<grid, kBlockThreads, 0, s>>>(b); break;
-    case RAFB200_F16: group_cast_kernel<ST, __half><<<grid, kBlockThreads, 0, s>>>(b); break;
-    default: group_cast_kernel<ST, __nv_bfloat16><<<grid, kBlockThreads, 0, s>>>(b); break;
+    case RAFB200_F32: return group_cast_any<ST, float>(k, src, dst, numel, s);
+    case RAFB200_F16: return group_cast_any<ST, __half>(k, src, dst, numel, s);
+    default: return group_cast_any<ST, __nv_bfloat16>(k, src, dst, numel, s);
   }
-  RAFB200_CUDA(cudaGetLastError());
-  return RAFB200_OK;
+}
+
+template <int CAP>
+static int group_copy_rows(int k, const void* const* src, void* const* dst, const int64_t* numel, int elem_size,
+                           cudaStream_t s) {
+  return for_each_group<CAP>(k, src, dst, numel, elem_size, kCopySpan, [&](const CopyRows<CAP>& r, int n, unsigned spans) {
+    RAFB200_CUDA(launch_dependent(group_copy_kernel<CAP>, spans, kBlockThreads, 0, s, r, n));
+    return (int)RAFB200_OK;
+  });
 }
 
 }  // namespace rafb200
@@ -615,22 +717,17 @@ int rafb200_group_cast(int k, const void* const* src, int src_dtype, void* const
   RAFB200_REQUIRE(k >= 0 && (k == 0 || (src && dst && numel)), "rafb200_group_cast: bad arguments");
   RAFB200_REQUIRE(dtype_valid(src_dtype) && dtype_valid(dst_dtype), "rafb200_group_cast: bad dtype");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  return for_each_batch(k, src, dst, numel, 1, 4, [&](const CopyBatch& b, dim3 grid) {
-    switch (src_dtype) {
-      case RAFB200_F32: return group_cast_dst<float>(b, grid, dst_dtype, s);
-      case RAFB200_F16: return group_cast_dst<__half>(b, grid, dst_dtype, s);
-      default: return group_cast_dst<__nv_bfloat16>(b, grid, dst_dtype, s);
-    }
-  });
+  switch (src_dtype) {
+    case RAFB200_F32: return group_cast_dst<float>(k, src, dst, dst_dtype, numel, s);
+    case RAFB200_F16: return group_cast_dst<__half>(k, src, dst, dst_dtype, numel, s);
+    default: return group_cast_dst<__nv_bfloat16>(k, src, dst, dst_dtype, numel, s);
+  }
 }
 
 static int group_copy(int k, const void* const* src, void* const* dst, const int64_t* numel,
                       int elem_size, cudaStream_t s) {
-  return for_each_batch(k, src, dst, numel, elem_size, 16, [&](const CopyBatch& b, dim3 grid) {
-    group_copy_kernel<<<grid, kBlockThreads, 0, s>>>(b);
-    RAFB200_CUDA(cudaGetLastError());
-    return (int)RAFB200_OK;
-  });
+  return k <= kFewRows ? group_copy_rows<kFewRows>(k, src, dst, numel, elem_size, s)
+                       : group_copy_rows<kMaxRows>(k, src, dst, numel, elem_size, s);
 }
 
 int rafb200_fuse_tensor(int k, const void* const* src, const int64_t* numel, const int64_t* offsets,

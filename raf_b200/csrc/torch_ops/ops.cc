@@ -26,6 +26,9 @@ namespace {
 struct {
   decltype(&rafb200_sgd_to) sgd_to;
   decltype(&rafb200_sgd_many) sgd_many;
+  decltype(&rafb200_group_cast) group_cast;
+  decltype(&rafb200_fuse_tensor) fuse_tensor;
+  decltype(&rafb200_defuse_tensor) defuse_tensor;
 } abi;
 
 PyObject* bind(PyObject*, PyObject* path) {
@@ -38,7 +41,10 @@ PyObject* bind(PyObject*, PyObject* path) {
     if (!fn) PyErr_Format(PyExc_ImportError, "%s has no %s", p, name);
     return fn != nullptr;
   };
-  if (!find(abi.sgd_to, "rafb200_sgd_to") || !find(abi.sgd_many, "rafb200_sgd_many")) return nullptr;
+  if (!find(abi.sgd_to, "rafb200_sgd_to") || !find(abi.sgd_many, "rafb200_sgd_many") ||
+      !find(abi.group_cast, "rafb200_group_cast") || !find(abi.fuse_tensor, "rafb200_fuse_tensor") ||
+      !find(abi.defuse_tensor, "rafb200_defuse_tensor"))
+    return nullptr;
   Py_RETURN_NONE;
 }
 
@@ -172,10 +178,158 @@ PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_RETURN_TRUE;
 }
 
+// The stream argument of an operator: an address, or None for the current stream.
+bool stream_of(PyObject* o, c10::DeviceIndex device, void** stream) {
+  if (o == Py_None) {
+    *stream = current_stream(device);
+    return true;
+  }
+  *stream = PyLong_AsVoidPtr(o);
+  if (!PyErr_Occurred()) return true;
+  PyErr_Clear();
+  return false;
+}
+
+// A non-empty list or tuple of dense CUDA tensors of one type: addresses and element counts.
+struct TensorRow {
+  std::vector<const at::Tensor*> t;
+  std::vector<const void*> ptr;
+  std::vector<int64_t> numel;
+  bool take(PyObject* seq, c10::DeviceIndex device) {
+    if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return false;
+    const Py_ssize_t k = PySequence_Fast_GET_SIZE(seq);
+    PyObject** items = PySequence_Fast_ITEMS(seq);
+    t.reserve(k);
+    ptr.reserve(k);
+    numel.reserve(k);
+    for (Py_ssize_t i = 0; i < k; ++i) {
+      const at::Tensor* x = plain(items[i], device);
+      if (!x || x->scalar_type() != (i ? t[0] : x)->scalar_type()) return false;
+      t.push_back(x);
+      ptr.push_back(x->const_data_ptr());
+      numel.push_back(x->numel());
+    }
+    return k > 0;
+  }
+};
+
+PyObject* wrapped_list(std::vector<at::Tensor>& ts) {
+  PyObject* out = PyList_New((Py_ssize_t)ts.size());
+  if (!out) return nullptr;
+  for (size_t i = 0; i < ts.size(); ++i) PyList_SET_ITEM(out, (Py_ssize_t)i, THPVariable_Wrap(std::move(ts[i])));
+  return out;
+}
+
+// group_cast(tensors, dtype code, stream) -> list
+PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  static const at::ScalarType types[] = {at::kFloat, at::kHalf, at::kBFloat16};
+  if (n != 3) return nothing();
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  TensorRow in;
+  void* stream = nullptr;
+  const long to = PyLong_AsLong(a[1]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return nothing();
+  }
+  if (to < 0 || to > 2 || !in.take(a[0], dev) || code_of(in.t[0]->scalar_type()) < 0 || !stream_of(a[2], dev, &stream))
+    return nothing();
+  std::vector<at::Tensor> outs;
+  std::vector<void*> dst;
+  outs.reserve(in.t.size());
+  dst.reserve(in.t.size());
+  for (const at::Tensor* x : in.t) {
+    outs.push_back(at::detail::empty_cuda(x->sizes(), types[to], x->device(), c10::nullopt));
+    dst.push_back(outs.back().mutable_data_ptr());
+  }
+  const int rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0]->scalar_type()), dst.data(), (int)to,
+                                in.numel.data(), stream);
+  if (rc != RAFB200_OK) return PyLong_FromLong(rc);
+  return wrapped_list(outs);
+}
+
+// fuse_tensor(tensors, stream) -> flat tensor
+PyObject* fuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 2) return nothing();
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  TensorRow in;
+  void* stream = nullptr;
+  if (!in.take(a[0], dev) || !stream_of(a[1], dev, &stream)) return nothing();
+  std::vector<int64_t> at_elem(in.t.size());
+  int64_t total = 0;
+  for (size_t i = 0; i < in.t.size(); ++i) {
+    at_elem[i] = total;
+    total += in.numel[i];
+  }
+  at::Tensor flat = at::detail::empty_cuda({total}, in.t[0]->scalar_type(), in.t[0]->device(), c10::nullopt);
+  const int rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(),
+                                 (int)in.t[0]->element_size(), flat.mutable_data_ptr(), stream);
+  if (rc != RAFB200_OK) return PyLong_FromLong(rc);
+  return THPVariable_Wrap(std::move(flat));
+}
+
+bool ints_of(PyObject* seq, std::vector<int64_t>* out) {
+  if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return false;
+  const Py_ssize_t k = PySequence_Fast_GET_SIZE(seq);
+  PyObject** items = PySequence_Fast_ITEMS(seq);
+  out->resize(k);
+  for (Py_ssize_t i = 0; i < k; ++i) {
+    if (!PyLong_CheckExact(items[i])) return false;
+    (*out)[i] = PyLong_AsLongLong(items[i]);
+    if ((*out)[i] < 0) {
+      PyErr_Clear();
+      return false;
+    }
+  }
+  return true;
+}
+
+// defuse_tensor(flat, sizes, shapes, shape_indices, stream) -> list
+PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 5) return nothing();
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  const at::Tensor* flat = plain(a[0], dev);
+  std::vector<int64_t> sizes, dims, ends, at_elem;
+  void* stream = nullptr;
+  if (!flat || !ints_of(a[1], &sizes) || !ints_of(a[2], &dims) || !ints_of(a[3], &ends) || ends.size() != sizes.size() ||
+      !stream_of(a[4], dev, &stream))
+    return nothing();
+  int64_t total = 0, from = 0;
+  for (size_t i = 0; i < sizes.size(); ++i) {
+    if (ends[i] < from || ends[i] > (int64_t)dims.size()) return nothing();
+    int64_t numel = 1;
+    for (int64_t d = from; d < ends[i]; ++d) numel *= dims[d];
+    if (numel != sizes[i]) return nothing();
+    at_elem.push_back(total);
+    total += sizes[i];
+    from = ends[i];
+  }
+  if (sizes.empty() || total > flat->numel()) return nothing();
+  std::vector<at::Tensor> outs;
+  std::vector<void*> dst;
+  outs.reserve(sizes.size());
+  dst.reserve(sizes.size());
+  from = 0;
+  for (size_t i = 0; i < sizes.size(); ++i) {
+    outs.push_back(at::detail::empty_cuda(at::IntArrayRef(dims.data() + from, (size_t)(ends[i] - from)),
+                                          flat->scalar_type(), flat->device(), c10::nullopt));
+    dst.push_back(outs.back().mutable_data_ptr());
+    from = ends[i];
+  }
+  const int rc = abi.defuse_tensor((int)sizes.size(), dst.data(), sizes.data(), at_elem.data(),
+                                   (int)flat->element_size(), flat->const_data_ptr(), stream);
+  if (rc != RAFB200_OK) return PyLong_FromLong(rc);
+  return wrapped_list(outs);
+}
+
 PyMethodDef kMethods[] = {
     {"bind", bind, METH_O, "use the C ABI of the loaded library at this path"},
     {"sgd", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd)), METH_FASTCALL, "raf.op.sgd"},
     {"sgd_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd_step)), METH_FASTCALL, "eager SGD, all parameters"},
+    {"group_cast", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(group_cast)), METH_FASTCALL, "raf.op.group_cast"},
+    {"fuse_tensor", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(fuse_tensor)), METH_FASTCALL, "raf.op.fuse_tensor"},
+    {"defuse_tensor", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(defuse_tensor)), METH_FASTCALL,
+     "raf.op.defuse_tensor"},
     {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_ops", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

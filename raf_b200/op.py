@@ -45,6 +45,11 @@ def stream_ptr(stream=None) -> int:
     return s.cuda_stream
 
 
+def _raw(stream):
+    """The address of a stream, or None: the native module looks up the current one itself."""
+    return None if stream is None else stream.cuda_stream
+
+
 # --------------------------------------------------------------------------- lists
 class TensorList:
     """Device-resident tensor list ([g..., p..., m..., v...] of raf.op.lans)."""
@@ -244,6 +249,11 @@ def cast(data, dtype, out=None, stream=None):
 def group_cast(tensor_list, dtype, stream=None):
     """raf.op.group_cast: one launch for the whole tuple."""
     dtype = torch_dtype(dtype)
+    r = _lib.ops().group_cast(tensor_list, _CODES.get(dtype, -1), _raw(stream))
+    if r.__class__ is list:
+        return r
+    if r is not None:
+        check(r)
     if not tensor_list:
         return []
     _check_cuda(*tensor_list)
@@ -259,6 +269,11 @@ def group_cast(tensor_list, dtype, stream=None):
 
 def fuse_tensor(tensor_list, stream=None):
     """raf.op.fuse_tensor: concatenate a tuple into one flat buffer."""
+    r = _lib.ops().fuse_tensor(tensor_list, _raw(stream))
+    if isinstance(r, torch.Tensor):
+        return r
+    if r is not None:
+        check(r)
     _check_cuda(*tensor_list)
     dtype = tensor_list[0].dtype
     numels = [t.numel() for t in tensor_list]
@@ -275,6 +290,11 @@ def fuse_tensor(tensor_list, stream=None):
 
 def defuse_tensor(data, sizes, shapes, shape_indices, stream=None):
     """raf.op.defuse_tensor (schema DefuseTensorArgs{data, sizes, shapes, shape_indices})."""
+    r = _lib.ops().defuse_tensor(data, sizes, shapes, shape_indices, _raw(stream))
+    if r.__class__ is list:
+        return r
+    if r is not None:
+        check(r)
     _check_cuda(data)
     outs, offsets, start = [], [], 0
     off = 0

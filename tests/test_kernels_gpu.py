@@ -527,3 +527,29 @@ def test_sgd_eager_step_one_launch_bit_exact(rb, count):
         assert bits_equal(to_numpy(x), ps[i]) and bits_equal(to_numpy(opt.state()[f"sgd.{i}.v"]), vs[i]), i
     if tied:
         assert bits_equal(to_numpy(opt.state()[f"sgd.{count}.v"]), v_tied)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.int8])
+@pytest.mark.parametrize("count", [3, 64, 65, 520])
+def test_fuse_defuse_misaligned(rb, dtype, count):
+    """Pieces of odd size, so that source and destination lie differently to 16 bytes, around the
+    bytes of a block's span and the table sizes of a launch."""
+    rng = np.random.default_rng(count)
+    es = torch.empty((), dtype=dtype).element_size()
+    span = 8192 // es
+    sizes = [int(s) for s in rng.choice([0, 1, 3, 15, 16, 17, 31, 33, span - 1, span, span + 1, 2 * span + 5], count)]
+    ts = [torch.from_numpy(rng.integers(-100, 100, s)).cuda().to(dtype) for s in sizes]
+    flat = rb.fuse_tensor(ts)
+    assert torch.equal(flat, torch.cat(ts))
+    back = rb.defuse_tensor(flat, sizes, sizes, list(range(1, count + 1)))
+    for a, b in zip(ts, back):
+        assert a.shape == b.shape and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("count", [1, 64, 65, 520])
+def test_group_cast_spans(rb, count):
+    rng = np.random.default_rng(count)
+    sizes = [int(s) for s in rng.choice([0, 1, 3, 4, 5, 4095, 4096, 4097, 9001], count)]
+    xs = [torch.from_numpy(rng.standard_normal(s + 1).astype(np.float32)).cuda()[i % 2:i % 2 + s] for i, s in enumerate(sizes)]
+    for x, y in zip(xs, rb.group_cast(xs, "bfloat16")):
+        assert y.dtype == torch.bfloat16 and bits_equal(to_numpy(y), O.cast(to_numpy(x), O.BF16))
