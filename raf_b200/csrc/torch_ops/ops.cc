@@ -8,7 +8,8 @@
 // returns its status as an int.
 #include <Python.h>
 
-#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -76,6 +77,21 @@ void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDA
 
 PyObject* nothing() { Py_RETURN_NONE; }
 
+// torch.empty on the current device, from torch's caching allocator: 0.5 us where the dispatched
+// form takes 1.3 us, and the list operators make up to hundreds of tensors a call.
+at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type) {
+  int64_t numel = 1;
+  for (int64_t d : sizes) numel *= d;
+  const int64_t bytes = numel * (int64_t)c10::elementSize(type);
+  c10::Allocator* alloc = c10::cuda::CUDACachingAllocator::get();
+  auto storage = c10::make_intrusive<c10::StorageImpl>(c10::StorageImpl::use_byte_size_t(), bytes,
+                                                       alloc->allocate((size_t)bytes), alloc, /*resizable=*/true);
+  at::Tensor t = at::detail::make_tensor_base<c10::TensorImpl>(std::move(storage), c10::DispatchKeySet(c10::DispatchKey::CUDA),
+                                                               c10::scalarTypeToTypeMeta(type));
+  t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
+  return t;
+}
+
 // sgd(x, dx, v, learning_rate, mu) -> (v1, x1)
 PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 5) return nothing();
@@ -91,8 +107,8 @@ PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat || code < 0 || x->sizes() != dx->sizes() ||
       x->sizes() != v->sizes())
     return nothing();
-  at::Tensor x1 = at::detail::empty_cuda(x->sizes(), at::kFloat, x->device(), c10::nullopt);
-  at::Tensor v1 = at::detail::empty_cuda(x->sizes(), at::kFloat, x->device(), c10::nullopt);
+  at::Tensor x1 = new_tensor(x->sizes(), at::kFloat);
+  at::Tensor v1 = new_tensor(x->sizes(), at::kFloat);
   const int rc = abi.sgd_to(x->const_data_ptr<float>(), dx->const_data_ptr(), code, v->const_data_ptr<float>(),
                                 x1.mutable_data_ptr<float>(), v1.mutable_data_ptr<float>(), x->numel(), (float)lr, (float)mu,
                                 current_stream(dev));
@@ -239,7 +255,7 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
   outs.reserve(in.t.size());
   dst.reserve(in.t.size());
   for (const at::Tensor* x : in.t) {
-    outs.push_back(at::detail::empty_cuda(x->sizes(), types[to], x->device(), c10::nullopt));
+    outs.push_back(new_tensor(x->sizes(), types[to]));
     dst.push_back(outs.back().mutable_data_ptr());
   }
   const int rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0]->scalar_type()), dst.data(), (int)to,
@@ -261,7 +277,7 @@ PyObject* fuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at_elem[i] = total;
     total += in.numel[i];
   }
-  at::Tensor flat = at::detail::empty_cuda({total}, in.t[0]->scalar_type(), in.t[0]->device(), c10::nullopt);
+  at::Tensor flat = new_tensor({total}, in.t[0]->scalar_type());
   const int rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(),
                                  (int)in.t[0]->element_size(), flat.mutable_data_ptr(), stream);
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
@@ -311,8 +327,7 @@ PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   dst.reserve(sizes.size());
   from = 0;
   for (size_t i = 0; i < sizes.size(); ++i) {
-    outs.push_back(at::detail::empty_cuda(at::IntArrayRef(dims.data() + from, (size_t)(ends[i] - from)),
-                                          flat->scalar_type(), flat->device(), c10::nullopt));
+    outs.push_back(new_tensor(at::IntArrayRef(dims.data() + from, (size_t)(ends[i] - from)), flat->scalar_type()));
     dst.push_back(outs.back().mutable_data_ptr());
     from = ends[i];
   }

@@ -129,26 +129,31 @@ class ZeroStep:
             pa([t.data_ptr() for t in v]) if v is not None else None))
         self._keep = (grads, params, p, m, v)
 
-    def step(self, hyper: Hyper, step: int, compute_stream=None, comm_stream=None):
+    def _streams(self, compute_stream, comm_stream) -> Tuple[int, int]:
+        """Addresses of the two streams of a step: the current one and the library's
+        communication stream unless given.  A world of one communicates nothing."""
+        cs = stream_ptr(compute_stream)
+        if comm_stream is not None:
+            return cs, comm_stream.cuda_stream
+        if self.plan.n_ranks == 1:
+            return cs, cs
         from .distributed import comm_stream as default_comm_stream
 
-        cs = compute_stream if compute_stream is not None else torch.cuda.current_stream()
-        ms = comm_stream if comm_stream is not None else default_comm_stream()
-        check(_lib.load().rafb200_zero_step(self.handle, C.byref(hyper), int(step), cs.cuda_stream,
-                                            ms.cuda_stream))
+        return cs, default_comm_stream().cuda_stream
+
+    def step(self, hyper: Hyper, step: int, compute_stream=None, comm_stream=None):
+        cs, ms = self._streams(compute_stream, comm_stream)
+        check(_lib.load().rafb200_zero_step(self.handle, C.byref(hyper), int(step), cs, ms))
 
     def step_host(self, hyper: Hyper, step: int, grads_host, params_host, compute_stream=None,
                   comm_stream=None):
         """Host-buffer form: gradients come from (pinned) host tensors, the updated
         model-dtype parameters are copied back into host tensors."""
-        from .distributed import comm_stream as default_comm_stream
-
-        cs = compute_stream if compute_stream is not None else torch.cuda.current_stream()
-        ms = comm_stream if comm_stream is not None else default_comm_stream()
+        cs, ms = self._streams(compute_stream, comm_stream)
         pa = _lib.ptr_array
         check(_lib.load().rafb200_zero_step_host(
             self.handle, C.byref(hyper), int(step), pa([t.data_ptr() for t in grads_host]),
-            pa([t.data_ptr() for t in params_host]), cs.cuda_stream, ms.cuda_stream))
+            pa([t.data_ptr() for t in params_host]), cs, ms))
 
     def launch_counts(self) -> Tuple[int, int]:
         a, b = C.c_int(), C.c_int()
