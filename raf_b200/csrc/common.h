@@ -184,5 +184,12 @@ struct rafb200_tensor_list_s {
 };
 
 namespace rafb200 {
+int sgd_list_items(rafb200_tensor_list_s* list, uint32_t first, uint32_t n, float learning_rate, float mu,
+                   float weight_decay, float grad_scale, cudaStream_t s);
+int adam_list_items(rafb200_tensor_list_s* list, uint32_t first, uint32_t n, int step, float learning_rate,
+                    float beta1, float beta2, float eps, int bias_correction, float weight_decay, int mode,
+                    float grad_scale, cudaStream_t s);
+// k byte copies in as few launches as the tables allow; either end may be page-locked host memory.
+int copy_many(int k, const void* const* src, void* const* dst, const int64_t* bytes, cudaStream_t s);
 int tensor_list_set_fuse(rafb200_tensor_list_s* l, const LansFuse& f, const int64_t* sym_off_bytes);
 }

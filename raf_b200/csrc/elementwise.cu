@@ -237,8 +237,9 @@ static int grid_for(uint32_t nitems, int device) {
   return (int)(nitems < cap ? (nitems ? nitems : 1) : cap);
 }
 
+// Items [first, first + n) of the list, all of them unless the caller cuts the list into groups.
 template <int NSTATE, typename Op, typename GT>
-static int launch_list_out(const rafb200_tensor_list_s* l, const Op& op, cudaStream_t s) {
+static int launch_list_out(const rafb200_tensor_list_s* l, const Op& op, uint32_t first, uint32_t n, cudaStream_t s) {
   if (l->fuse.fuse_rs) {
     const int grid = grid_for(l->n_items, l->device);
     switch (l->out_dtype) {
@@ -255,28 +256,29 @@ static int launch_list_out(const rafb200_tensor_list_s* l, const Op& op, cudaStr
     RAFB200_CUDA(cudaGetLastError());
     return RAFB200_OK;
   }
-  const unsigned blocks = l->n_items * kSpansPerChunk;
+  const unsigned blocks = n * kSpansPerChunk;
+  const Item* items = l->dev_items + first;
   switch (l->out_dtype) {
     case RAFB200_F32:
-      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, float, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, l->dev_items, op));
+      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, float, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, items, op));
       break;
     case RAFB200_F16:
-      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, __half, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, l->dev_items, op));
+      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, __half, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, items, op));
       break;
     default:
-      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, __nv_bfloat16, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, l->dev_items, op));
+      RAFB200_CUDA(launch_dependent(update_list_kernel<NSTATE, GT, __nv_bfloat16, Op>, blocks, kBlockThreads, 0, s, l->dev_desc, items, op));
       break;
   }
   return RAFB200_OK;
 }
 
 template <int NSTATE, typename Op>
-static int launch_list(const rafb200_tensor_list_s* l, const Op& op, cudaStream_t s) {
-  if (l->n_items == 0) return RAFB200_OK;
+static int launch_list(const rafb200_tensor_list_s* l, const Op& op, uint32_t first, uint32_t n, cudaStream_t s) {
+  if (n == 0) return RAFB200_OK;
   switch (l->g_dtype) {
-    case RAFB200_F32: return launch_list_out<NSTATE, Op, float>(l, op, s);
-    case RAFB200_F16: return launch_list_out<NSTATE, Op, __half>(l, op, s);
-    default: return launch_list_out<NSTATE, Op, __nv_bfloat16>(l, op, s);
+    case RAFB200_F32: return launch_list_out<NSTATE, Op, float>(l, op, first, n, s);
+    case RAFB200_F16: return launch_list_out<NSTATE, Op, __half>(l, op, first, n, s);
+    default: return launch_list_out<NSTATE, Op, __nv_bfloat16>(l, op, first, n, s);
   }
 }
 
@@ -592,6 +594,48 @@ static int group_copy_rows(int k, const void* const* src, void* const* dst, cons
   });
 }
 
+static int group_copy(int k, const void* const* src, void* const* dst, const int64_t* numel, int elem_size,
+                      cudaStream_t s) {
+  return k <= kFewRows ? group_copy_rows<kFewRows>(k, src, dst, numel, elem_size, s)
+                       : group_copy_rows<kMaxRows>(k, src, dst, numel, elem_size, s);
+}
+
+int copy_many(int k, const void* const* src, void* const* dst, const int64_t* bytes, cudaStream_t s) {
+  return group_copy(k, src, dst, bytes, 1, s);
+}
+
+// The list's update on part of its work items (item i = 4096 elements, tensor by tensor).
+int sgd_list_items(rafb200_tensor_list_s* list, uint32_t first, uint32_t n, float learning_rate, float mu,
+                   float weight_decay, float grad_scale, cudaStream_t s) {
+  RAFB200_REQUIRE(list->bound, "rafb200_sgd_list: bind the tensor list first");
+  SgdOp op{learning_rate, mu, weight_decay, grad_scale};
+  return launch_list<1>(list, op, first, n, s);
+}
+
+int adam_list_items(rafb200_tensor_list_s* list, uint32_t first, uint32_t n, int step, float learning_rate,
+                    float beta1, float beta2, float eps, int bias_correction, float weight_decay, int mode,
+                    float grad_scale, cudaStream_t s) {
+  RAFB200_REQUIRE(list->bound && list->has_v, "rafb200_adam: bind g, p, m and v first");
+  RAFB200_REQUIRE(step >= 1, "rafb200_adam: step counts from 1");
+  AdamOp op;
+  op.lr = learning_rate;
+  op.beta1 = beta1;
+  op.beta2 = beta2;
+  op.beta3 = 1 - beta1;
+  op.one_minus_beta2 = 1 - beta2;
+  op.eps = eps;
+  bias_corrections(beta1, beta2, step, bias_correction, &op.bc1, &op.bc2);
+  op.wd = weight_decay;
+  op.gscale = grad_scale;
+  op.mode = mode;
+  // the branch-free form of AdamOp::vec: see the ranges there
+  op.y1 = 1.0f / op.bc1;
+  op.y2 = 1.0f / op.bc2;
+  auto within = [](float x, float lo, float hi) { return x >= lo && x <= hi; };
+  op.fast = within(op.bc1, 0x1p-20f, 1.0f) && within(op.bc2, 0x1p-20f, 1.0f) && within(eps, 0x1p-40f, 1.0f);
+  return launch_list<2>(list, op, first, n, s);
+}
+
 }  // namespace rafb200
 
 using namespace rafb200;
@@ -673,36 +717,18 @@ int rafb200_sgd_many(int k, float* const* x, const void* const* dx, int dx_dtype
 int rafb200_sgd_list(rafb200_tensor_list_t list, float learning_rate, float mu,
                      float weight_decay, float grad_scale, void* stream) {
   RAFB200_REQUIRE(list, "rafb200_sgd_list: NULL list");
-  RAFB200_REQUIRE(list->bound, "rafb200_sgd_list: bind the tensor list first");
-  SgdOp op{learning_rate, mu, weight_decay, grad_scale};
-  return launch_list<1>(list, op, static_cast<cudaStream_t>(stream));
+  return sgd_list_items(list, 0, list->n_items, learning_rate, mu, weight_decay, grad_scale,
+                        static_cast<cudaStream_t>(stream));
 }
 
 int rafb200_adam(rafb200_tensor_list_t list, int step, const float* step_dev,
                  float learning_rate, float beta1, float beta2, float eps, int bias_correction,
                  float weight_decay, int mode, float grad_scale, void* stream) {
   RAFB200_REQUIRE(list, "rafb200_adam: NULL list");
-  RAFB200_REQUIRE(list->bound && list->has_v, "rafb200_adam: bind g, p, m and v first");
   RAFB200_REQUIRE(step_dev == nullptr,
                   "rafb200_adam: a device-resident step is only supported by rafb200_lans");
-  RAFB200_REQUIRE(step >= 1, "rafb200_adam: step counts from 1");
-  AdamOp op;
-  op.lr = learning_rate;
-  op.beta1 = beta1;
-  op.beta2 = beta2;
-  op.beta3 = 1 - beta1;
-  op.one_minus_beta2 = 1 - beta2;
-  op.eps = eps;
-  bias_corrections(beta1, beta2, step, bias_correction, &op.bc1, &op.bc2);
-  op.wd = weight_decay;
-  op.gscale = grad_scale;
-  op.mode = mode;
-  // the branch-free form of AdamOp::vec: see the ranges there
-  op.y1 = 1.0f / op.bc1;
-  op.y2 = 1.0f / op.bc2;
-  auto within = [](float x, float lo, float hi) { return x >= lo && x <= hi; };
-  op.fast = within(op.bc1, 0x1p-20f, 1.0f) && within(op.bc2, 0x1p-20f, 1.0f) && within(eps, 0x1p-40f, 1.0f);
-  return launch_list<2>(list, op, static_cast<cudaStream_t>(stream));
+  return adam_list_items(list, 0, list->n_items, step, learning_rate, beta1, beta2, eps, bias_correction, weight_decay,
+                         mode, grad_scale, static_cast<cudaStream_t>(stream));
 }
 
 int rafb200_cast(const void* src, int src_dtype, void* dst, int dst_dtype, int64_t numel,
@@ -722,12 +748,6 @@ int rafb200_group_cast(int k, const void* const* src, int src_dtype, void* const
     case RAFB200_F16: return group_cast_dst<__half>(k, src, dst, dst_dtype, numel, s);
     default: return group_cast_dst<__nv_bfloat16>(k, src, dst, dst_dtype, numel, s);
   }
-}
-
-static int group_copy(int k, const void* const* src, void* const* dst, const int64_t* numel,
-                      int elem_size, cudaStream_t s) {
-  return k <= kFewRows ? group_copy_rows<kFewRows>(k, src, dst, numel, elem_size, s)
-                       : group_copy_rows<kMaxRows>(k, src, dst, numel, elem_size, s);
 }
 
 int rafb200_fuse_tensor(int k, const void* const* src, const int64_t* numel, const int64_t* offsets,

@@ -4,6 +4,7 @@
 //   -> ONE all-gather  ->  unpack (row blocks -> the caller's parameter tensors).
 // Collectives run on the communication stream, kernels on the compute stream.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <memory>
 
@@ -60,6 +61,20 @@ struct Bucket {
   Item* dev_rs_items = nullptr;
   Item* dev_ag_items = nullptr;
   uint32_t n_rs_items = 0, n_ag_items = 0;
+};
+
+// Host-buffer form on one rank: what is copied in, updated and copied out together.  For SGD and
+// Adam a group is a run of the list's work items - tensors are cut where a group ends - for LANS
+// it is whole tensors with a list of their own.
+struct HostPiece {
+  int tensor;
+  int64_t lo, hi;  // elements
+};
+struct HostGroup {
+  std::vector<HostPiece> pieces;
+  uint32_t first_item = 0, n_items = 0;  // SGD / Adam
+  int bucket = -1;                       // LANS: index into hbuckets
+  cudaEvent_t h2d_done = nullptr, out_ready = nullptr;
 };
 
 // Copies every segment; 16-byte accesses when both ends of a segment are aligned,
@@ -140,9 +155,10 @@ struct rafb200_zero_s {
   int n = 1, rank = 0;
   int g_dtype = 0, param_dtype = 0, optimizer = 0;
   std::vector<rafb200::Bucket> buckets;
-  // world of one, host-buffer form: one list per plan bucket so that the copy of bucket b+1
-  // from the host, the update of bucket b and the copy of bucket b-1 to the host overlap
-  std::vector<rafb200::Bucket> hbuckets;
+  // world of one, host-buffer form: the copy of group j+1 from the host, the update of group j
+  // and the copy of group j-1 to the host overlap
+  std::vector<rafb200::HostGroup> hgroups;
+  std::vector<rafb200::Bucket> hbuckets;  // LANS: the lists of the groups
   cudaStream_t h2d_stream = nullptr, d2h_stream = nullptr;
   cudaEvent_t ev_d2h_done = nullptr;
   char* g_flat = nullptr;  // all buckets' gradient buffers, one allocation (n > 1)
@@ -190,6 +206,55 @@ struct rafb200_zero_s {
   void* fused_ws = nullptr;
   size_t fused_ws_bytes = 0;
 };
+
+namespace rafb200 {
+
+// The groups of the host-buffer form.  The copies out trail the copies in by one group, and every
+// group costs about 8 us beyond its bytes (at 50 GB/s, 400 KB) while both directions are busy: the
+// sum is least with groups of sqrt(bytes * 400 KB).  Measured on 102 MB each way (2.13 ms as one
+// plain copy per direction): 2 MiB 3.14 ms, 8 MiB 2.56 ms, 34 MB 2.80 ms; groups that grow and
+// shrink gain nothing, because the lag is that of the largest.  LANS takes whole tensors.
+static void make_host_groups(rafb200_zero_s* z) {
+  const rafb200_plan_s& plan = z->plan;
+  const bool whole = z->optimizer == RAFB200_OPT_LANS;
+  const int64_t wide = std::max(dtype_size(z->g_dtype), dtype_size(z->param_dtype));
+  const double bytes = std::min(32e6, std::max(1e6, std::sqrt((double)plan.total * (double)wide * 400e3)));
+  const int64_t target = std::max<int64_t>(1, (int64_t)bytes / wide / kChunkElems) * kChunkElems;  // elements
+  int64_t room = 0;
+  uint32_t item = 0;
+  for (int i = 0; i < plan.k; ++i) {
+    const int64_t n = plan.numel[i];
+    for (int64_t at = 0; at < n;) {
+      if (room <= 0 || (whole && !z->hgroups.back().pieces.empty() && n > room)) {
+        z->hgroups.emplace_back();
+        z->hgroups.back().first_item = item;
+        room = target;
+      }
+      HostGroup& g = z->hgroups.back();
+      int64_t take = n - at;
+      if (!whole && take > room) take = (room + kChunkElems - 1) / kChunkElems * kChunkElems;
+      if (take > n - at) take = n - at;
+      g.pieces.push_back(HostPiece{i, at, at + take});
+      const uint32_t items = (uint32_t)((take + kChunkElems - 1) / kChunkElems);
+      g.n_items += items;
+      item += items;
+      room -= take;
+      at += take;
+    }
+  }
+  if (!whole) return;
+  if (z->hgroups.size() < 2) {  // one group: the list of the whole plan
+    if (!z->hgroups.empty()) z->hgroups[0].bucket = -1;
+    return;
+  }
+  for (HostGroup& g : z->hgroups) {
+    g.bucket = (int)z->hbuckets.size();
+    z->hbuckets.emplace_back();
+    for (const HostPiece& p : g.pieces) z->hbuckets.back().tensors.push_back(p.tensor);
+  }
+}
+
+}  // namespace rafb200
 
 using namespace rafb200;
 
@@ -288,6 +353,9 @@ int rafb200_zero_destroy(rafb200_zero_t z) {
                       (void*)b.dev_rs_items, (void*)b.dev_ag_items})
       if (ptr) cudaFree(ptr);
   }
+  for (auto& g : z->hgroups)
+    for (cudaEvent_t e : {g.h2d_done, g.out_ready})
+      if (e) cudaEventDestroy(e);
   if (z->g_flat && !z->symmetric) rafb200_comm_free(z->comm, z->g_flat);
   if (z->p_flat && !z->symmetric) rafb200_comm_free(z->comm, z->p_flat);
   if (z->dev_err) cudaFree(z->dev_err);
@@ -337,22 +405,7 @@ int rafb200_zero_create(rafb200_plan_t plan, rafb200_comm_t comm, int g_dtype, i
     const int nb = (z->n == 1) ? (k > 0 ? 1 : 0) : plan->nbuckets;
     z->buckets.resize(nb);
     for (int i = 0; i < k; ++i) z->buckets[z->n == 1 ? 0 : plan->bucket_of[i]].tensors.push_back(i);
-    if (z->n == 1 && k > 1) {
-      // Host-buffer form on one rank: groups of about 16 Mi elements (32-64 MB over PCIe, a
-      // few ms each way), small enough that the first copy in and the last copy out, which
-      // nothing overlaps, stay short.
-      constexpr int64_t kHostGroupElems = 16ll << 20;
-      int64_t run = 0;
-      for (int i = 0; i < k; ++i) {
-        if (z->hbuckets.empty() || (run > 0 && run + plan->numel[i] > kHostGroupElems)) {
-          z->hbuckets.emplace_back();
-          run = 0;
-        }
-        z->hbuckets.back().tensors.push_back(i);
-        run += plan->numel[i];
-      }
-      if (z->hbuckets.size() < 2) z->hbuckets.clear();
-    }
+    if (z->n == 1) make_host_groups(z);
     int64_t flat_elems = 0;
     for (auto* set : {&z->buckets, &z->hbuckets}) {
       for (auto& b : *set) {
@@ -379,6 +432,10 @@ int rafb200_zero_create(rafb200_plan_t plan, rafb200_comm_t comm, int g_dtype, i
       }
       if (rc != RAFB200_OK) break;
     }
+    for (auto& g : z->hgroups)
+      for (cudaEvent_t* e : {&g.h2d_done, &g.out_ready})
+        if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess)
+          rc = set_error(RAFB200_CUDA_ERROR, "rafb200_zero_create: cannot create events");
     if (rc != RAFB200_OK) break;
     if (cudaStreamCreateWithFlags(&z->h2d_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&z->d2h_stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -773,80 +830,70 @@ static int step_impl(rafb200_zero_t z, const rafb200_hyper* h, int step, void* c
   const float gscale = h->grad_scale * ((h->average && z->n > 1) ? 1.0f / (float)z->n : 1.0f);
   const int gs = dtype_size(z->g_dtype), ps = dtype_size(z->param_dtype);
   const bool host = grads_host != nullptr;
-  std::vector<Bucket>& bl = (z->n == 1 && host && !z->hbuckets.empty()) ? z->hbuckets : z->buckets;
-  const int nb = (int)bl.size();
-  if (host) {
-    // Every copy from the host is queued up front, bucket by bucket, behind whatever the
-    // compute stream still does with the gradient buffers.
-    RAFB200_CUDA(cudaEventRecord(z->ev_start, cs));
-    RAFB200_CUDA(cudaStreamWaitEvent(z->h2d_stream, z->ev_start, 0));
-    RAFB200_CUDA(cudaStreamWaitEvent(z->d2h_stream, z->ev_start, 0));
-    for (auto& b : bl) {
-      // Tensors that follow one another in host AND device memory, inside ranges the caller
-      // declared to be single allocations, travel as one copy: a caller that keeps its
-      // gradients (parameters) in one arena per side pays one copy per bucket and direction
-      // instead of one per tensor.  (A copy must not span two allocations, however close.)
-      const char *run_src = nullptr;
-      char* run_dst = nullptr;
-      size_t run = 0;
-      auto flush = [&]() -> int {
-        if (run) RAFB200_CUDA(cudaMemcpyAsync(run_dst, run_src, run, cudaMemcpyHostToDevice, z->h2d_stream));
-        run = 0;
-        return RAFB200_OK;
-      };
-      for (int i : b.tensors) {
-        const size_t bytes = (size_t)z->plan.numel[i] * gs;
-        if (!bytes) continue;
-        const char* src = static_cast<const char*>(grads_host[i]);
-        char* dst = static_cast<char*>(z->grads[i]);
-        if (run && src == run_src + run && dst == run_dst + run && z->in_one_arena(run_src, src + bytes) &&
-            z->in_one_arena(run_dst, dst + bytes)) {
-          run += bytes;
-          continue;
-        }
-        if (int rc = flush()) return rc;
-        run_src = src;
-        run_dst = dst;
-        run = bytes;
-      }
-      if (int rc = flush()) return rc;
-      RAFB200_CUDA(cudaEventRecord(b.h2d_done, z->h2d_stream));
+  const int nb = (int)z->buckets.size();
+  // Small pieces that stand alone go through a kernel that reads (writes) the page-locked host
+  // memory itself, all of a group in one launch: a copy of its own costs each about 8 us on the
+  // copy engine, which moves 400 KB in that time.
+  struct Small {
+    std::vector<const void*> src;
+    std::vector<void*> dst;
+    std::vector<int64_t> bytes;
+  };
+  constexpr size_t kSmallBytes = 256 << 10;
+  auto device_view = [](const void* host_ptr) -> void* {  // of page-locked memory; NULL for other memory
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host_ptr) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
     }
-  }
-  auto copy_out = [&](Bucket& b) -> int {  // after the last kernel of bucket b on the compute stream
-    if (!host) return RAFB200_OK;
-    RAFB200_CUDA(cudaEventRecord(b.out_ready, cs));
-    RAFB200_CUDA(cudaStreamWaitEvent(z->d2h_stream, b.out_ready, 0));
-    const char* run_src = nullptr;
-    char* run_dst = nullptr;
-    size_t run = 0;
-    auto flush = [&]() -> int {
-      if (run) RAFB200_CUDA(cudaMemcpyAsync(run_dst, run_src, run, cudaMemcpyDeviceToHost, z->d2h_stream));
-      run = 0;
+    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+  };
+  // Pieces that follow one another in host AND device memory, inside ranges the caller declared to
+  // be single allocations, travel as one copy: a caller that keeps its gradients (parameters) in
+  // one arena per side pays one copy per group and direction instead of one per tensor.  (A copy
+  // must not span two allocations, however close.)
+  struct Run {
+    const char* src = nullptr;
+    char* dst = nullptr;
+    size_t bytes = 0;
+  };
+  auto add_copy = [&](Run& r, const char* src, char* dst, size_t bytes, cudaMemcpyKind kind, cudaStream_t s,
+                      Small* small = nullptr) -> int {
+    if (bytes && r.bytes && src == r.src + r.bytes && dst == r.dst + r.bytes && z->in_one_arena(r.src, src + bytes) &&
+        z->in_one_arena(r.dst, dst + bytes)) {
+      r.bytes += bytes;
       return RAFB200_OK;
-    };
-    for (int i : b.tensors) {
-      // what leaves: the whole parameter, or (host_output 1) the rows this rank owns
-      int64_t lo = 0, hi = z->plan.numel[i];
-      if (z->host_output == 1 && z->n > 1) {
-        lo = std::min<int64_t>(hi, (int64_t)z->rank * z->plan.shard_elems[i]);
-        hi = std::min<int64_t>(hi, lo + z->plan.shard_elems[i]);
-      }
-      const size_t bytes = (size_t)(hi - lo) * ps;
-      if (!bytes) continue;
-      const char* src = static_cast<const char*>(z->params[i]) + (size_t)lo * ps;
-      char* dst = static_cast<char*>(params_host[i]) + (size_t)lo * ps;
-      if (run && src == run_src + run && dst == run_dst + run && z->in_one_arena(run_src, src + bytes) &&
-          z->in_one_arena(run_dst, dst + bytes)) {
-        run += bytes;
-        continue;
-      }
-      if (int rc = flush()) return rc;
-      run_src = src;
-      run_dst = dst;
-      run = bytes;
     }
-    return flush();
+    if (bytes == 0 && src) return RAFB200_OK;  // an empty piece; src NULL: end of the run
+    if (r.bytes) {
+      const bool in = kind == cudaMemcpyHostToDevice;
+      void* mapped = small && r.bytes < kSmallBytes ? device_view(in ? r.src : r.dst) : nullptr;
+      if (mapped) {
+        small->src.push_back(in ? mapped : r.src);
+        small->dst.push_back(in ? r.dst : mapped);
+        small->bytes.push_back((int64_t)r.bytes);
+      } else {
+        RAFB200_CUDA(cudaMemcpyAsync(r.dst, r.src, r.bytes, kind, s));
+      }
+    }
+    r = Run{src, dst, bytes};
+    if (!src && small && !small->src.empty()) {  // the end of a group
+      if (int rc = copy_many((int)small->src.size(), small->src.data(), small->dst.data(), small->bytes.data(), s)) return rc;
+      small->src.clear();
+      small->dst.clear();
+      small->bytes.clear();
+    }
+    return RAFB200_OK;
+  };
+  auto copy_in = [&](int i, int64_t lo, int64_t hi, Run& r, Small* small = nullptr) -> int {
+    return add_copy(r, static_cast<const char*>(grads_host[i]) + (size_t)lo * gs,
+                    static_cast<char*>(z->grads[i]) + (size_t)lo * gs, (size_t)(hi - lo) * gs, cudaMemcpyHostToDevice,
+                    z->h2d_stream, small);
+  };
+  auto copy_back = [&](int i, int64_t lo, int64_t hi, Run& r, Small* small = nullptr) -> int {
+    return add_copy(r, static_cast<const char*>(z->params[i]) + (size_t)lo * ps,
+                    static_cast<char*>(params_host[i]) + (size_t)lo * ps, (size_t)(hi - lo) * ps, cudaMemcpyDeviceToHost,
+                    z->d2h_stream, small);
   };
   auto finish = [&]() -> int {  // the compute stream ends the step for the caller
     if (!host) return RAFB200_OK;
@@ -854,15 +901,72 @@ static int step_impl(rafb200_zero_t z, const rafb200_hyper* h, int step, void* c
     RAFB200_CUDA(cudaStreamWaitEvent(cs, z->ev_d2h_done, 0));
     return RAFB200_OK;
   };
-  if (z->n == 1) {
-    for (auto& b : bl) {
-      if (host) RAFB200_CUDA(cudaStreamWaitEvent(cs, b.h2d_done, 0));
+  if (host) {
+    // behind whatever the compute stream still does with the gradient buffers
+    RAFB200_CUDA(cudaEventRecord(z->ev_start, cs));
+    RAFB200_CUDA(cudaStreamWaitEvent(z->h2d_stream, z->ev_start, 0));
+    RAFB200_CUDA(cudaStreamWaitEvent(z->d2h_stream, z->ev_start, 0));
+  }
+  if (z->n == 1 && !host) {
+    for (auto& b : z->buckets) {
       int rc = run_update(z, b, h, step, gscale, cs);
       if (rc != RAFB200_OK) return rc;
-      if ((rc = copy_out(b)) != RAFB200_OK) return rc;
+    }
+    return RAFB200_OK;
+  }
+  if (z->n == 1) {
+    Small small;
+    for (HostGroup& g : z->hgroups) {
+      int rc = RAFB200_OK;
+      Run in, out;
+      for (const HostPiece& p : g.pieces)
+        if ((rc = copy_in(p.tensor, p.lo, p.hi, in, &small)) != RAFB200_OK) return rc;
+      if ((rc = add_copy(in, nullptr, nullptr, 0, cudaMemcpyHostToDevice, z->h2d_stream, &small)) != RAFB200_OK) return rc;
+      RAFB200_CUDA(cudaEventRecord(g.h2d_done, z->h2d_stream));
+      RAFB200_CUDA(cudaStreamWaitEvent(cs, g.h2d_done, 0));
+      rafb200_tensor_list_s* whole = z->buckets[0].list;
+      if (z->optimizer == RAFB200_OPT_SGD)
+        rc = sgd_list_items(whole, g.first_item, g.n_items, h->learning_rate, h->mu, h->weight_decay, gscale, cs);
+      else if (z->optimizer == RAFB200_OPT_ADAM)
+        rc = adam_list_items(whole, g.first_item, g.n_items, step, h->learning_rate, h->beta1, h->beta2, h->eps,
+                             h->bias_correction, h->weight_decay, h->mode, gscale, cs);
+      else
+        rc = run_update(z, g.bucket >= 0 ? z->hbuckets[g.bucket] : z->buckets[0], h, step, gscale, cs);
+      if (rc != RAFB200_OK) return rc;
+      RAFB200_CUDA(cudaEventRecord(g.out_ready, cs));
+      RAFB200_CUDA(cudaStreamWaitEvent(z->d2h_stream, g.out_ready, 0));
+      for (const HostPiece& p : g.pieces)
+        if ((rc = copy_back(p.tensor, p.lo, p.hi, out, &small)) != RAFB200_OK) return rc;
+      if ((rc = add_copy(out, nullptr, nullptr, 0, cudaMemcpyDeviceToHost, z->d2h_stream, &small)) != RAFB200_OK) return rc;
     }
     return finish();
   }
+  if (host) {
+    // every copy from the host is queued up front, bucket by bucket
+    for (auto& b : z->buckets) {
+      Run in;
+      for (int i : b.tensors)
+        if (int rc = copy_in(i, 0, z->plan.numel[i], in)) return rc;
+      if (int rc = add_copy(in, nullptr, nullptr, 0, cudaMemcpyHostToDevice, z->h2d_stream)) return rc;
+      RAFB200_CUDA(cudaEventRecord(b.h2d_done, z->h2d_stream));
+    }
+  }
+  auto copy_out = [&](Bucket& b) -> int {  // after the last kernel of bucket b on the compute stream
+    if (!host) return RAFB200_OK;
+    RAFB200_CUDA(cudaEventRecord(b.out_ready, cs));
+    RAFB200_CUDA(cudaStreamWaitEvent(z->d2h_stream, b.out_ready, 0));
+    Run out;
+    for (int i : b.tensors) {
+      // what leaves: the whole parameter, or (host_output 1) the rows this rank owns
+      int64_t lo = 0, hi = z->plan.numel[i];
+      if (z->host_output == 1) {
+        lo = std::min<int64_t>(hi, (int64_t)z->rank * z->plan.shard_elems[i]);
+        hi = std::min<int64_t>(hi, lo + z->plan.shard_elems[i]);
+      }
+      if (int rc = copy_back(i, lo, hi, out)) return rc;
+    }
+    return add_copy(out, nullptr, nullptr, 0, cudaMemcpyDeviceToHost, z->d2h_stream);
+  };
   // (the host-buffer form keeps the bucketed pipeline: there the copies from and to the host
   // bound the step, and they overlap with the buckets' kernels)
   if (z->fused && !host && z->symmetric && (z->optimizer != RAFB200_OPT_LANS || h->normalize_grad) && z->stage_mask == 31) {

@@ -94,3 +94,53 @@ def test_zero_step_host_buffers():
         assert rel_err(to_numpy(tp[i]), p[i]) < 1e-5
         assert torch.equal(params_host[i], params_dev[i].cpu())
     z.close()
+
+
+@pytest.mark.parametrize("optimizer", ["sgd", "adam", "lans"])
+@pytest.mark.parametrize("arena", [False, True])
+def test_zero_step_host_groups(optimizer, arena):
+    """Enough elements for several groups of the host-buffer form: tensors cut where a group ends
+    (SGD, Adam), ending next to a work item's 4096 elements, empty and tiny ones between them."""
+    from raf_b200 import distributed as dist
+    from raf_b200.zero import Plan, ZeroStep, make_hyper
+
+    sizes = [700001, 0, 3, 262144, 1, 1200033, 4096, 8191]
+    plan = Plan([(n,) for n in sizes], 1, 0, 1 << 20)
+    z = ZeroStep(plan, dist.get_communicator(), "float32", "float32", optimizer)
+    rng = np.random.default_rng(17)
+    at = np.concatenate([[0], np.cumsum([(n + 3) // 4 * 4 for n in sizes])])
+
+    def tensors(device, fill=None):
+        buf = torch.zeros(int(at[-1]), device=device) if device == "cuda" else torch.zeros(int(at[-1])).pin_memory()
+        if arena:
+            z.declare_arena(buf)
+        ts = [buf[int(o):int(o) + n] for o, n in zip(at, sizes)]
+        for t, x in zip(ts, fill or []):
+            t.copy_(torch.from_numpy(x))
+        return ts
+
+    p = [(rng.standard_normal(n) * 0.02).astype(np.float32) for n in sizes]
+    m, v = [np.zeros(n, np.float32) for n in sizes], [np.zeros(n, np.float32) for n in sizes]
+    tp, tm, tv = tensors("cuda", p), tensors("cuda"), tensors("cuda")
+    z.bind(tensors("cuda"), tp, tp, tm, tv)
+    hyper = make_hyper(optimizer, learning_rate=1e-2, mu=0.9)
+    for step in (1, 2):
+        g = [(rng.standard_normal(n) * 1e-3).astype(np.float32) for n in sizes]
+        back = tensors("cpu")
+        z.step_host(hyper, step, tensors("cpu", g), back)
+        torch.cuda.synchronize()
+        if optimizer == "sgd":
+            for i in range(len(p)):
+                O.sgd(p[i], g[i], m[i], 1e-2, 0.9)
+        elif optimizer == "adam":
+            for i in range(len(p)):
+                O.adam(g[i], p[i], m[i], v[i], step, 1e-2, 0.9, 0.999, 1e-6, 1, 0.0, 1)
+        else:
+            O.lans(g, p, m, v, step, 1e-2, 0.9, 0.999, 1e-6, 1, 0.0, 1, 1, 1)
+        for i in range(len(p)):
+            if optimizer == "lans":
+                assert rel_err(to_numpy(tp[i]), p[i]) < 1e-5 and rel_err(to_numpy(tm[i]), m[i]) < 1e-5
+            else:
+                assert bits_equal(to_numpy(tp[i]), p[i]) and bits_equal(to_numpy(tm[i]), m[i])
+            assert torch.equal(back[i], tp[i].cpu())
+    z.close()
