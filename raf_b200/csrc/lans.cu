@@ -29,14 +29,13 @@
 // remains for every earlier item without one), and a tensor has fewer parked items in a list
 // than the list has cells: the bounded waits below cannot deadlock.
 //
-// Roles inside a block (640 threads):
+// Roles inside a block (704 threads):
 //   warps 0-15  four consumer groups of four warps; group q serves the slots s with
-//               s % 4 == q.  The warps of a group take turns in the bookkeeping after an
-//               operation: free the slot or cell, take the slot's next item from its
-//               mailbox and start it (bulk copies + first operation).
+//               s % 4 == q.  A warp that has a chunk's values in registers lets go of the slot
+//               and never waits for the other warps of its group.
 //   warps 16,17 prefetchers, one per list: a lane per mailbox resolves the items ahead of
 //               their use (item -> descriptor -> the norms its first operation needs are
-//               final -> a cell if it parks -> mailbox).
+//               final -> mailbox).  All they wait for is global memory.
 //   warp 18     parker: owns the tensor-memory allocation; lane c polls the norm words of the
 //               tensor whose chunk is parked in cell c and queues the chunk's second half;
 //               lanes that wait for the same tensor share one load.
@@ -44,6 +43,16 @@
 //               precision) to the tensor's accumulators, counts arrivals; the last
 //               arrival takes the square root and publishes the norm together with its
 //               "final" bit in one word.
+//   warps 20,21 turnover, one per list: hand out the cells, start the next item of a slot that
+//               is free (bulk copies + first operation) and turn filled cells into parked ones,
+//               emptied cells into free ones.  All they touch is shared memory.
+// What bounds it: the latency of the chain cell -> copies -> stage 1 -> norms -> stage 2, because a
+// chunk holds its cell all that time and a block runs ahead of the slowest one by its cells alone.
+// Every link that ran between round trips to global memory, or on a consumer warp that first waited for
+// the rest of its group, lengthened it (measured: prefetcher pass 2.2 us, bookkeeping of an operation
+// 2 us of a consumer warp, publisher pass 2.6 us).  With those links on shared-memory-only warps and two
+// buffers of sums a slot: BERT-large, fp16, 2.22 -> 2.06 ms; a shard of eight 272 -> 252 us; fp32
+// gradients, a shard of four, 600 -> 495 us.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -61,7 +70,7 @@ void bias_corrections(float beta1, float beta2, int step, int bias_correction, f
                       float* bc2);
 
 constexpr uint32_t kOpA = 0, kOpB = 1, kOpBP = 2, kOpC = 3, kOpCP = 4, kOpEnd = 7;
-constexpr unsigned kErrWaitG = 1, kErrWaitN = 2, kErrRing = 3, kErrData = 4, kErrDone = 5;
+constexpr unsigned kErrWaitG = 1, kErrWaitN = 2, kErrRing = 3, kErrData = 4;
 
 struct LansParams {
   const TensorDesc* descs;
@@ -298,6 +307,15 @@ __device__ __forceinline__ bool ring_wait(uint32_t bar, uint32_t parity, LansHea
 }
 
 
+// Bounded wait that an error does not cut short: what a block waits for before it leaves.
+__device__ __forceinline__ void drain_wait(uint32_t bar, uint32_t parity, uint64_t wait_ns) {
+  const uint64_t t0 = global_ns();
+  while (!mbar_try_wait(bar, parity))
+    if (global_ns() - t0 > wait_ns) return;
+}
+
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
 // ---- kernel geometry ---------------------------------------------------------------
 constexpr int kGroups = 4;                       // consumer groups per block
 constexpr int kGroupThreads = 128;               // four warps
@@ -305,10 +323,11 @@ constexpr int kConsumerWarps = kGroups * 4;      // 16
 constexpr int kPrefWarp = kConsumerWarps;        // 16, 17: resolve the block's items ahead of their use
 constexpr int kParkWarp = kConsumerWarps + 2;    // 18: finishes parked chunks
 constexpr int kPubWarp = kConsumerWarps + 3;     // 19: adds partial sums to the tensors' accumulators
-constexpr int kLansThreads = (kConsumerWarps + 4) * 32;  // 640
+constexpr int kTurnWarp = kConsumerWarps + 4;    // 20, 21: start items, turn slots and cells over
+constexpr int kLansThreads = (kConsumerWarps + 6) * 32;  // 704; up to 24 warps have the same 80 registers a thread
 constexpr int kQueueDepth = 64;                  // > slots per group + parked cells + end marker
 constexpr int kMail = 64;                        // mailboxes of a block: kMailboxes per slot
-constexpr uint32_t kMbEmpty = 0, kMbFull = 1, kMbTaking = 2, kMbIdle = 3;
+constexpr uint32_t kMbEmpty = 0, kMbFull = 1, kMbWants = 2;  // kMbWants: complete but for its cell
 constexpr uint32_t kSeqBits = 11, kSeqMask = (1u << kSeqBits) - 1u;  // see partition_lans_items
 constexpr int kBVecs = kLansElems / (kGroupThreads * kVec);  // 2 vectors per thread per chunk
 static_assert(kBVecs * kGroupThreads * kVec == kLansElems, "a chunk is whole passes of a group");
@@ -342,14 +361,12 @@ static_assert(sizeof(RedSlot) == 64, "RedSlot is 64 bytes");
 
 // Block-wide control words in shared memory.
 struct LansCtrl {
-  uint32_t done_items;  // items of this block that have finished
-  uint32_t mb_state[64]; // mailbox kMailboxes * slot + round % kMailboxes, see kMb*
+  uint32_t done_items;   // items of this block that have finished
+  uint32_t mb_state[kMail];  // mailbox kMailboxes * slot + round % kMailboxes, see kMb*
   uint32_t tail[kGroups];
-  uint32_t item_cnt[16], pub_cnt[16], op_cnt[16];  // per slot: parities of its barriers
-  uint32_t cell_free;    // cells nobody holds
   uint32_t cell_parked;  // cells whose chunk waits for its tensor's norms
   uint32_t tmem_base;    // address the allocation returned
-  uint32_t cellop_cnt[32], cell_grp[32];  // per cell: parity of its barrier, group that parked it
+  uint32_t cell_grp[32];  // per cell: group that parks its chunk
 };
 
 // What the second half of a parked item needs: where p and the parameter copy go.
@@ -380,12 +397,13 @@ struct LansGeo {
   static constexpr int kMetaOff = kSmemCellOff + kLansSmemCells * kSmemCellBytes;
   static constexpr int kMailOff = kMetaOff + kSlots * (int)sizeof(SlotMeta);
   static constexpr int kRedOff = kMailOff + kMail * (int)sizeof(SlotMeta);
-  static constexpr int kQueueOff = kRedOff + kSlots * (int)sizeof(RedSlot);
+  static constexpr int kQueueOff = kRedOff + 2 * kSlots * (int)sizeof(RedSlot);
   static constexpr int kCellOff = kQueueOff + kGroups * kQueueDepth * 16;
   static constexpr int kCtrlOff = kCellOff + kLansCells * (int)sizeof(CellMeta);
   static constexpr int kBarOff = (kCtrlOff + (int)sizeof(LansCtrl) + 15) & ~15;
-  // barriers: data, done, redfull, redempty per slot; queue entries; end of consumers; per cell
-  static constexpr int kNumBars = 4 * kSlots + kGroups * kQueueDepth + 1 + kLansCells;
+  // barriers: data, done per slot; redfull, redempty per buffer of sums (two a slot); queue entries; end
+  // of consumers; per cell
+  static constexpr int kNumBars = 6 * kSlots + kGroups * kQueueDepth + 1 + kLansCells;
   static constexpr int kTotal = kBarOff + kNumBars * 8;
   static_assert(kTotal <= 232448, "fits the 227 KB of shared memory a block may use");
 };
@@ -410,8 +428,8 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
   const uint32_t bar_data = smem_u32(smem + L::kBarOff);
   const uint32_t bar_done = bar_data + S * 8;
   const uint32_t bar_redfull = bar_done + S * 8;
-  const uint32_t bar_redempty = bar_redfull + S * 8;
-  const uint32_t bar_queue = bar_redempty + S * 8;
+  const uint32_t bar_redempty = bar_redfull + 2 * S * 8;
+  const uint32_t bar_queue = bar_redempty + 2 * S * 8;
   const uint32_t bar_end = bar_queue + kGroups * kQueueDepth * 8;
   const uint32_t bar_cell = bar_end + 8;
   const uint32_t data_base = smem_u32(smem);
@@ -426,15 +444,15 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
     for (int s = 0; s < S; ++s) {
       mbar_init(bar_data + 8 * s, 1);      // whoever starts the item (+ transaction bytes)
       mbar_init(bar_done + 8 * s, 4);      // the four warps of the slot's group
-      mbar_init(bar_redfull + 8 * s, 4);
-      mbar_init(bar_redempty + 8 * s, 1);  // the publisher
+      for (int b = 2 * s; b < 2 * s + 2; ++b) {
+        mbar_init(bar_redfull + 8 * b, 4);
+        mbar_init(bar_redempty + 8 * b, 1);  // the publisher
+      }
     }
     for (int q = 0; q < kGroups * kQueueDepth; ++q) mbar_init(bar_queue + 8 * q, 1);
     mbar_init(bar_end, kConsumerWarps);
     for (int c = 0; c < kLansCells; ++c) mbar_init(bar_cell + 8 * c, 4);
     memset(ctrl, 0, sizeof(LansCtrl));
-    for (int q = 0; q < S; ++q) ctrl->mb_state[kMailboxes * q] = kMbIdle;  // every slot waits for its first item
-    ctrl->cell_free = (1u << kLansCells) - 1u;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -459,74 +477,13 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
   const uint64_t pol_keep = make_policy_keep(), pol_stream = make_policy_stream();
 
   // Hands one entry of a group's queue to that group.  Called by a single thread.
-  // `slot` is a shared-memory slot, or - for kOpCP - a tensor-memory cell.
-  auto push_op = [&](uint32_t slot, uint32_t op, uint32_t dpar, uint32_t rpar, float cs, float rm, float rg) {
-    const uint32_t grp = (op == kOpCP) ? ld_shared_volatile(&ctrl->cell_grp[slot]) : (slot & 3u);
-    const uint32_t opar = atomicAdd(op == kOpCP ? &ctrl->cellop_cnt[slot] : &ctrl->op_cnt[slot], 1u) & 1u;
+  // `slot` is a shared-memory slot, or - for kOpCP - a cell; `pars` = parity of the data barrier,
+  // buffer of sums and its parity in bits 0 .. 2.
+  auto push_op = [&](uint32_t grp, uint32_t slot, uint32_t op, uint32_t pars, float cs, float rm, float rg) {
     const uint32_t tail = atomicAdd(&ctrl->tail[grp], 1u);
     const uint32_t qi = grp * kQueueDepth + (tail % kQueueDepth);
-    s_queue[qi] = make_uint4(op | (slot << 3) | (dpar << 8) | (rpar << 9) | (opar << 10), __float_as_uint(cs),
-                             __float_as_uint(rm), __float_as_uint(rg));
+    s_queue[qi] = make_uint4(op | (slot << 3) | (pars << 8), __float_as_uint(cs), __float_as_uint(rm), __float_as_uint(rg));
     mbar_arrive(bar_queue + 8 * qi);
-  };
-  // Every slot has two mailboxes for its next items (rounds of the slot alternate between
-  // them), filled by the prefetcher.  A mailbox is EMPTY, FULL, being TAKEN, or the slot sits
-  // IDLE in front of it: then whoever fills it starts the item himself.
-  //
-  // Starts the item in mailbox `h` of slot `slot`: copies it into the slot's description,
-  // issues the bulk copies and queues the item's first operation.  Called by a single thread.
-  auto start_from_mailbox = [&](uint32_t slot, uint32_t h) {
-    const uint4* src = reinterpret_cast<const uint4*>(&s_mail[kMailboxes * slot + h]);
-    uint4* dst = reinterpret_cast<uint4*>(&s_meta[slot]);
-    const uint4 e0 = src[0], e1 = src[1], e2 = src[2], e3 = src[3];
-    dst[0] = e0;
-    dst[1] = e1;
-    dst[2] = e2;
-    dst[3] = e3;
-    __threadfence_block();
-    *reinterpret_cast<volatile uint32_t*>(&ctrl->mb_state[kMailboxes * slot + h]) = kMbEmpty;
-    const uint32_t op = e2.w >> 30, nbulk = (e2.z >> kLansNBits) & ((1u << kLansNBits) - 1u);
-    const uint32_t dpar = atomicAdd(&ctrl->item_cnt[slot], 1u) & 1u;
-    const uint32_t my_data = bar_data + 8 * slot;
-    if (nbulk > 0) {
-      const char* gsrc = reinterpret_cast<const char*>(((uint64_t)e0.y << 32) | e0.x);
-      const char* psrc = reinterpret_cast<const char*>(((uint64_t)e0.w << 32) | e0.z);
-      const char* msrc = reinterpret_cast<const char*>(((uint64_t)e1.y << 32) | e1.x);
-      const char* vsrc = reinterpret_cast<const char*>(((uint64_t)e1.w << 32) | e1.z);
-      const uint32_t gb = nbulk * (uint32_t)sizeof(GT), fb = nbulk * 4u;
-      const uint32_t dstaddr = data_base + slot * L::kSlotBytes;
-      if (op == kOpA) {
-        mbar_arrive_expect_tx(my_data, gb);
-        tma_load_1d(dstaddr, gsrc, gb, my_data, pol_keep);  // stage 1 reads it again soon
-      } else {
-        mbar_arrive_expect_tx(my_data, gb + 3u * fb);
-        // a streamed chunk is read once more by its update item soon after: keep it in L2;
-        // a parked chunk and the update item's own reads are the last use of the lines
-        const uint64_t pol = (op == kOpB) ? pol_keep : pol_stream;
-        tma_load_1d(dstaddr, gsrc, gb, my_data, pol);
-        tma_load_1d(dstaddr + L::kGBytes, psrc, fb, my_data, pol);
-        tma_load_1d(dstaddr + L::kGBytes + L::kFBytes, msrc, fb, my_data, pol);
-        tma_load_1d(dstaddr + L::kGBytes + 2 * L::kFBytes, vsrc, fb, my_data, pol);
-      }
-    } else {
-      mbar_arrive(my_data);
-    }
-    uint32_t rpar = 0;
-    if (op != kOpC) rpar = atomicAdd(&ctrl->pub_cnt[slot], 1u) & 1u;
-    if (op == kOpBP) rpar |= (atomicAdd(&ctrl->cellop_cnt[e2.z >> (2 * kLansNBits)], 1u) & 1u) << 2;  // lands in bit 11
-    push_op(slot, op, dpar, rpar, __uint_as_float(e3.y), __uint_as_float(e3.z), __uint_as_float(e3.w));
-  };
-  // The slot has run empty: take its next item if the prefetcher has it ready, else leave
-  // word that the slot is idle.  Called by a single thread that owns the slot.
-  auto take_next = [&](uint32_t slot) {
-    const uint32_t h = ld_shared_volatile(&ctrl->item_cnt[slot]) % kMailboxes;
-    uint32_t* stp = &ctrl->mb_state[kMailboxes * slot + h];
-    uint32_t old = atomicCAS(stp, kMbFull, kMbTaking);
-    if (old != kMbFull) {
-      old = atomicCAS(stp, kMbEmpty, kMbIdle);
-      if (old == kMbFull) old = atomicCAS(stp, kMbFull, kMbTaking);
-    }
-    if (old == kMbFull) start_from_mailbox(slot, h);
   };
 
   if (warp == kPrefWarp || warp == kPrefWarp + 1) {
@@ -535,28 +492,25 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
     // parity with S_h slots runs the entries j, j + S_h, j + 2 S_h, ... of its list.  Eight lanes
     // prepare them in turn (round r goes to mailbox r % 8): item -> descriptor of its tensor (kept
     // while the tensor stays the same) -> the norms the item's first operation needs are
-    // final -> a tensor-memory cell if the item parks -> the slot's mailbox.
-    enum : uint32_t { F_ITEM, F_DESC, F_NORM, F_CELL, F_WRITE, F_DONE };
-    // Two warps: warp w serves the slots s with s % 2 == w, kMailboxes lanes per slot,
-    // and hands out its own half of the tensor-memory cells.
+    // final -> the slot's mailbox.  Every pass of the loop is a round trip to global memory (about 2 us
+    // under load); what has to be quick - cells, starting items - is the turnover warps' work.
+    enum : uint32_t { F_ITEM, F_DESC, F_NORM, F_WRITE, F_DONE };
+    // Two warps: warp w serves the slots s with s % 2 == w, kMailboxes lanes per slot.
     const uint32_t pw = (uint32_t)(warp - kPrefWarp);
     constexpr uint32_t kJMask = (1u << L::kJBits) - 1u;
     const uint32_t slot = 2u * ((uint32_t)lane & kJMask) + pw, half = (uint32_t)lane >> L::kJBits;
-    const uint32_t my_cells = pw == 0 ? ((1u << ((kLansCells + 1) / 2)) - 1u)
-                                      : (((1u << kLansCells) - 1u) & ~((1u << ((kLansCells + 1) / 2)) - 1u));
     const uint32_t list_lo = P.block_off[2 * blockIdx.x + pw];
     const uint32_t my_n = P.block_off[2 * blockIdx.x + pw + 1] - list_lo;
     const uint32_t S_h = ((uint32_t)S + 1u - pw) / 2u;  // slots of my parity
     uint32_t e = ((uint32_t)lane & kJMask) + S_h * half;  // my entry of the list
     uint32_t st = (slot < (uint32_t)S && e < my_n) ? (uint32_t)F_ITEM : (uint32_t)F_DONE;
-    uint32_t tp = 0, chunk = 0, seq = 0, my_t = 0xffffffffu, my_cell = 0;
+    uint32_t tp = 0, chunk = 0, seq = 0, my_t = 0xffffffffu;
     uint4 d0 = make_uint4(0, 0, 0, 0), d1 = d0, d2 = d0, d3 = d0, nrm = d0;
     bool have_g = false, have_n = false;
     float cs = s1.gscale, rm = 0.f, rg = 0.f;
     uint64_t t_enter = 0;
     const bool normalize = s1.normalize != 0;
     int failed = 0;
-    uint32_t g_base = 0, g_mask = 0;
     for (uint32_t iter = 1;; ++iter) {
       const uint32_t st_in = st;
       // ---- global requests of this iteration, all issued before any is used ----
@@ -615,52 +569,13 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
       if (st == F_NORM) {
         const bool need_g = normalize && kind != kKindA;
         const bool need_n = kind == kKindCs;
-        if ((!need_g || have_g) && (!need_n || have_n)) st = (kind == kKindBCp) ? (uint32_t)F_CELL : (uint32_t)F_WRITE;
-      }
-      // ---- tensor-memory cells ----
-      // `seq` numbers the parked items of this block in list order.  An item may take a cell
-      // out of turn as long as a free cell remains for every earlier item that has none yet:
-      // then no item ever holds a cell that an earlier one is waiting for.  g_base = lowest
-      // number without a cell, bit i of g_mask = number g_base + i has one (warp-uniform).
-      {
-        const uint32_t off = (seq - g_base) & kSeqMask;
-        const bool asks = st == F_CELL && off < 32u;
-        uint32_t cand = asks ? (1u << off) : 0u;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cand |= __shfl_xor_sync(0xffffffffu, cand, o);
-        uint32_t free_cells = 0;
-        if (lane == 0) free_cells = ld_shared_volatile(&ctrl->cell_free) & my_cells;
-        free_cells = __shfl_sync(0xffffffffu, free_cells, 0);
-        uint32_t nfree = (uint32_t)__popc(free_cells), newly = 0;
-        for (uint32_t c = cand; c != 0 && nfree > 0; c &= c - 1u) {
-          const uint32_t o = (uint32_t)__ffs(c) - 1u;
-          const uint32_t earlier_without = o - (uint32_t)__popc((g_mask | newly) & ((1u << o) - 1u));
-          if (nfree - 1u < earlier_without) break;  // later numbers have at least as many before them
-          newly |= 1u << o;
-          --nfree;
-        }
-        if (newly) {
-          if (asks && ((newly >> off) & 1u)) {
-            my_cell = __fns(free_cells, 0, __popc(newly & ((1u << off) - 1u)) + 1);
-            st = F_WRITE;
-          }
-          uint32_t taken = (st == F_WRITE && asks && ((newly >> off) & 1u)) ? (1u << my_cell) : 0u;
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) taken |= __shfl_xor_sync(0xffffffffu, taken, o);
-          if (lane == 0) atomicAnd(&ctrl->cell_free, ~taken);
-          g_mask |= newly;
-          while (g_mask & 1u) {
-            g_mask >>= 1;
-            ++g_base;
-          }
-          __syncwarp();
-        }
+        if ((!need_g || have_g) && (!need_n || have_n)) st = F_WRITE;
       }
       // ---- hand the item to its slot ----
       if (st == F_WRITE) {
         const uint32_t mb = kMailboxes * slot + half;
         const uint32_t mbs = ld_shared_volatile(&ctrl->mb_state[mb]);
-        if (mbs == kMbEmpty || mbs == kMbIdle) {
+        if (mbs == kMbEmpty) {
           const char* dg = reinterpret_cast<const char*>(((uint64_t)d0.y << 32) | d0.x);
           float* dp = reinterpret_cast<float*>(((uint64_t)d0.w << 32) | d0.z);
           float* dm = reinterpret_cast<float*>(((uint64_t)d1.y << 32) | d1.x);
@@ -685,25 +600,14 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
           mt.m = dm + start;
           mt.v = dv + start;
           mt.out = dout ? dout + start * (int64_t)sizeof(OT) : nullptr;
-          mt.n_nbulk = (uint32_t)n | ((uint32_t)nbulk << kLansNBits) | ((op == kOpBP ? my_cell : 0u) << (2 * kLansNBits));
+          mt.n_nbulk = (uint32_t)n | ((uint32_t)nbulk << kLansNBits);
           mt.tensor_op = my_t | (op << 30);
           mt.nparts = (uint32_t)((numel + per - 1) / per);
           mt.cs = (op == kOpA) ? s1.gscale : cs;
-          mt.ratio_m = rm;
+          mt.ratio_m = op == kOpBP ? __uint_as_float(seq) : rm;  // a parked item is ranked by its number
           mt.ratio_g = rg;
-          if (op == kOpBP) {
-            CellMeta& cm = s_cell[my_cell];
-            cm.p = dp + start;
-            cm.out = mt.out;
-            cm.n_nbulk = (uint32_t)n | ((uint32_t)nbulk << kLansNBits);
-            cm.tensor = my_t;
-          }
           __threadfence_block();
-          if (atomicCAS(&ctrl->mb_state[mb], kMbEmpty, kMbFull) == kMbIdle) {
-            // the slot has been waiting for this item: start it from here
-            *reinterpret_cast<volatile uint32_t*>(&ctrl->mb_state[mb]) = kMbTaking;
-            start_from_mailbox(slot, half);
-          }
+          *reinterpret_cast<volatile uint32_t*>(&ctrl->mb_state[mb]) = op == kOpBP ? kMbWants : kMbFull;
           e += kMailboxes * S_h;
           st = e < my_n ? (uint32_t)F_ITEM : (uint32_t)F_DONE;
         }
@@ -712,11 +616,11 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
       // ---- bounded waits, errors, end ----
       if ((iter & 31u) == 0) {
         const uint64_t now = global_ns();
-        if (st == F_NORM || st == F_CELL) {
+        if (st == F_NORM) {
           if (t_enter == 0) {
             t_enter = now;
           } else if (now - t_enter > P.wait_ns) {
-            if (atomicCAS(&P.hdr->error, 0u, (kind == kKindCs || st == F_CELL) ? kErrWaitN : kErrWaitG) == 0u)
+            if (atomicCAS(&P.hdr->error, 0u, kind == kKindCs ? kErrWaitN : kErrWaitG) == 0u)
               P.hdr->error_item = list_lo + e;
           }
         }
@@ -732,7 +636,6 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
     // ================================= parker =================================
     // Lane c looks after cell c: queues the second half of the chunk parked there when the
     // tensor's norms are final.
-    const bool active = lane < S;
     const uint32_t bit = 1u << lane;
     uint64_t t_parked = 0;
     int failed = 0;
@@ -753,7 +656,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
         const float a = (umn != 0.0f && pn != 0.0f) ? mul(P.lr, fdiv(pn, umn)) : P.lr;
         const float b2 = (ugn != 0.0f && pn != 0.0f) ? mul(P.lr, fdiv(pn, ugn)) : P.lr;
         atomicAnd(&ctrl->cell_parked, ~bit);
-        push_op((uint32_t)lane, kOpCP, 0, 0, 0.f, -mul(a, s1.beta1), -mul(b2, s1.beta3));
+        push_op(ld_shared_volatile(&ctrl->cell_grp[lane]), (uint32_t)lane, kOpCP, 0, 0.f, -mul(a, s1.beta1), -mul(b2, s1.beta3));
         t_parked = 0;
       }
       __syncwarp();
@@ -779,11 +682,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
       s_queue[qi] = make_uint4(kOpEnd, 0, 0, 0);
       mbar_arrive(bar_queue + 8 * qi);
     }
-    ring_wait(bar_end, 0, P.hdr, kErrRing, 0x3000u, P.wait_ns);
-    if (active) {
-      const uint32_t items = ld_shared_volatile(&ctrl->item_cnt[lane]);
-      if (items > 0) ring_wait(bar_data + 8 * lane, (items - 1u) & 1u, P.hdr, kErrData, (uint32_t)lane, P.wait_ns);
-    }
+    drain_wait(bar_end, 0, P.wait_ns);
     // every consumer warp has left (or the bounded wait above gave up): give the tensor
     // memory back
     __syncwarp();
@@ -791,65 +690,220 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
     return;
   }
 
+  if (warp == kTurnWarp || warp == kTurnWarp + 1) {
+    // ================================ turnover ================================
+    // One warp per list, on shared memory alone.  Lane j looks after the j-th slot of the list's
+    // parity, lane c after the c-th of the list's cells, and every lane after one mailbox.  A
+    // slot that its group has let go of takes the next item from its mailbox; a cell is parked
+    // when its group has filled it and free again when its group has emptied it.
+    const uint32_t tw = (uint32_t)(warp - kTurnWarp);
+    const uint32_t S_h = ((uint32_t)S + 1u - tw) / 2u;  // slots of my parity
+    const uint32_t cell0 = tw == 0 ? 0u : (uint32_t)(kLansCells + 1) / 2u;
+    const uint32_t n_cells = tw == 0 ? (uint32_t)(kLansCells + 1) / 2u : (uint32_t)kLansCells / 2u;
+    const uint32_t my_n = P.block_off[2 * blockIdx.x + tw + 1] - P.block_off[2 * blockIdx.x + tw];
+    const uint32_t slot = 2u * (uint32_t)lane + tw;
+    const bool has_slot = (uint32_t)lane < S_h, has_cell = (uint32_t)lane < n_cells;
+    constexpr uint32_t kJMask = (1u << L::kJBits) - 1u;
+    const uint32_t mb_slot = 2u * ((uint32_t)lane & kJMask) + tw;
+    const bool has_mb = mb_slot < (uint32_t)S;
+    const uint32_t mb = kMailboxes * mb_slot + ((uint32_t)lane >> L::kJBits);
+    bool idle = has_slot;
+    uint32_t rounds = 0, pubs = 0, cur_op = 0;  // of my slot: items started, sums published, operation
+    uint32_t cell_phase = 0;                    // of my cell: even = to be filled, odd = to be emptied
+    uint32_t free_cells = (1u << n_cells) - 1u, g_base = 0, g_mask = 0, finished = 0;
+    uint64_t t_wants = 0;
+    int failed = 0;
+    for (uint32_t iter = 1; finished < my_n; ++iter) {
+      // ---- what the groups have let go of ----
+      const bool let_go = has_slot && !idle && mbar_test(bar_done + 8 * slot, (rounds - 1u) & 1u);
+      const bool turned = has_cell && mbar_test(bar_cell + 8 * (cell0 + (uint32_t)lane), cell_phase & 1u);
+      const unsigned filled = __ballot_sync(0xffffffffu, turned && !(cell_phase & 1u));
+      const unsigned emptied = __ballot_sync(0xffffffffu, turned && (cell_phase & 1u));
+      // an item is finished with its slot, a parked one with its cell
+      const unsigned n_done =
+          (unsigned)__popc(emptied) + (unsigned)__popc(__ballot_sync(0xffffffffu, let_go && cur_op != kOpBP));
+      cell_phase += turned ? 1u : 0u;
+      idle = idle || let_go;
+      free_cells |= emptied;
+      finished += n_done;
+      if (filled | n_done) {
+        __syncwarp();
+        if (lane == 0) {
+          __threadfence_block();
+          if (filled) atomicOr(&ctrl->cell_parked, filled << cell0);
+          if (n_done) atomicAdd(&ctrl->done_items, n_done);
+        }
+      }
+      // ---- cells ----
+      // The parked items of a list are numbered in list order.  An item may take a cell out of turn as
+      // long as a free cell remains for every earlier item that has none yet: then no item ever
+      // holds a cell that an earlier one is waiting for.  g_base = lowest number without a cell,
+      // bit i of g_mask = number g_base + i has one (all warp-uniform).
+      const bool wants = has_mb && ld_shared_volatile(&ctrl->mb_state[mb]) == kMbWants;
+      const bool any_wants = __any_sync(0xffffffffu, wants);
+      uint32_t newly = 0;
+      if (any_wants && free_cells) {
+        __threadfence_block();
+        const uint32_t off = wants ? (__float_as_uint(s_mail[mb].ratio_m) - g_base) & kSeqMask : 32u;
+        const bool asks = off < 32u;
+        const uint32_t cand = __reduce_or_sync(0xffffffffu, asks ? 1u << off : 0u);
+        uint32_t nfree = (uint32_t)__popc(free_cells);
+        for (uint32_t c = cand; c != 0 && nfree > 0; c &= c - 1u) {
+          const uint32_t o = (uint32_t)__ffs(c) - 1u;
+          const uint32_t earlier_without = o - (uint32_t)__popc((g_mask | newly) & ((1u << o) - 1u));
+          if (nfree - 1u < earlier_without) break;  // later numbers have at least as many before them
+          newly |= 1u << o;
+          --nfree;
+        }
+        if (newly) {
+          uint32_t taken = 0;
+          if (asks && ((newly >> off) & 1u)) {
+            uint32_t f = free_cells;  // the n-th number served takes the n-th free cell
+            for (uint32_t n = (uint32_t)__popc(newly & ((1u << off) - 1u)); n > 0; --n) f &= f - 1u;
+            taken = f & (0u - f);
+            s_mail[mb].n_nbulk |= (cell0 + (uint32_t)__ffs(f) - 1u) << (2 * kLansNBits);
+            __threadfence_block();
+            *reinterpret_cast<volatile uint32_t*>(&ctrl->mb_state[mb]) = kMbFull;
+          }
+          free_cells &= ~__reduce_or_sync(0xffffffffu, taken);
+          g_mask |= newly;
+          while (g_mask & 1u) {
+            g_mask >>= 1;
+            ++g_base;
+          }
+        }
+      }
+      __syncwarp();
+      // ---- start the next item of an idle slot ----
+      const uint32_t next = kMailboxes * slot + rounds % kMailboxes;
+      const bool starts = idle && ld_shared_volatile(&ctrl->mb_state[next]) == kMbFull;
+      if (starts) {
+        __threadfence_block();
+        const uint4* src = reinterpret_cast<const uint4*>(&s_mail[next]);
+        const uint4 e0 = src[0], e1 = src[1], e2 = src[2], e3 = src[3];
+        const uint32_t op = e2.w >> 30, nbulk = (e2.z >> kLansNBits) & ((1u << kLansNBits) - 1u);
+        const uint32_t my_data = bar_data + 8 * slot;
+        if (nbulk > 0) {
+          const char* gsrc = reinterpret_cast<const char*>(((uint64_t)e0.y << 32) | e0.x);
+          const char* psrc = reinterpret_cast<const char*>(((uint64_t)e0.w << 32) | e0.z);
+          const char* msrc = reinterpret_cast<const char*>(((uint64_t)e1.y << 32) | e1.x);
+          const char* vsrc = reinterpret_cast<const char*>(((uint64_t)e1.w << 32) | e1.z);
+          const uint32_t gb = nbulk * (uint32_t)sizeof(GT), fb = nbulk * 4u;
+          const uint32_t dstaddr = data_base + slot * L::kSlotBytes;
+          // what is read again soon stays in L2: a gradient for its norm (stage 1 follows) and a
+          // streamed chunk's first reading; a parked chunk and the second reading are the last use
+          const uint64_t pol = (op == kOpA || op == kOpB) ? pol_keep : pol_stream;
+          mbar_arrive_expect_tx(my_data, op == kOpA ? gb : gb + 3u * fb);
+          tma_load_1d(dstaddr, gsrc, gb, my_data, pol);
+          if (op != kOpA) {
+            tma_load_1d(dstaddr + L::kGBytes, psrc, fb, my_data, pol);
+            tma_load_1d(dstaddr + L::kGBytes + L::kFBytes, msrc, fb, my_data, pol);
+            tma_load_1d(dstaddr + L::kGBytes + 2 * L::kFBytes, vsrc, fb, my_data, pol);
+          }
+        } else {
+          mbar_arrive(my_data);
+        }
+        uint4* dst = reinterpret_cast<uint4*>(&s_meta[slot]);
+        dst[0] = e0;
+        dst[1] = e1;
+        dst[2] = e2;
+        dst[3] = e3;
+        if (op == kOpBP) {
+          const uint32_t cell = e2.z >> (2 * kLansNBits);
+          uint4* cm = reinterpret_cast<uint4*>(&s_cell[cell]);  // p, out, counts, tensor
+          cm[0] = make_uint4(e0.z, e0.w, e2.x, e2.y);
+          cm[1] = make_uint4(e2.z & ((1u << (2 * kLansNBits)) - 1u), e2.w & kTensorMask, 0u, 0u);
+          ctrl->cell_grp[cell] = slot & 3u;
+        }
+        __threadfence_block();
+        *reinterpret_cast<volatile uint32_t*>(&ctrl->mb_state[next]) = kMbEmpty;
+        uint32_t pars = rounds & 1u;
+        if (op != kOpC) pars |= ((pubs & 1u) << 1) | (((pubs >> 1) & 1u) << 2);
+        pubs += op != kOpC ? 1u : 0u;
+        ++rounds;
+        cur_op = op;
+        idle = false;
+        push_op(slot & 3u, slot, op, pars, __uint_as_float(e3.y), __uint_as_float(e3.z), __uint_as_float(e3.w));
+      }
+      __syncwarp();
+      // ---- bounded waits, errors ----
+      if ((iter & 255u) == 0) {
+        if (any_wants && !newly) {
+          const uint64_t now = global_ns();
+          if (t_wants == 0) {
+            t_wants = now;
+          } else if (now - t_wants > P.wait_ns && lane == 0) {
+            if (atomicCAS(&P.hdr->error, 0u, kErrWaitN) == 0u) P.hdr->error_item = 0x40000000u | g_base;
+          }
+        }
+        if (*reinterpret_cast<volatile unsigned*>(&P.hdr->error) != 0) failed = 1;
+        if (__any_sync(0xffffffffu, failed != 0)) break;
+      }
+      if (newly) t_wants = 0;
+    }
+    // after an error: no copy of this list's slots may still be in flight when the block ends
+    if (has_slot && rounds > 0) drain_wait(bar_data + 8 * slot, (rounds - 1u) & 1u, P.wait_ns);
+    return;
+  }
+
   if (warp == kPubWarp) {
     // =============================== publisher ===============================
-    const bool active = lane < S;
-    uint32_t n_seen = 0;  // publications of this lane's slot read so far
+    // One lane per buffer of sums.  Items of the same tensor and kind that completed since the
+    // last look go out as one update of the tensor's accumulators (the lowest of their lanes adds
+    // them up and sends it): the atomic operations on one address take about 1 ns each whatever the number
+    // of blocks, so one per item would cost a tensor of 64 Mi elements 200 us more than this.
+    const bool active = lane < 2 * S;
+    uint32_t n_seen = 0;  // publications read from this lane's buffer
     for (;;) {
       const bool end = mbar_test(bar_end, 0);  // every consumer warp has left (checked first)
       const bool ready = active && mbar_test(bar_redfull + 8 * lane, n_seen & 1u);
-      double q0 = 0.0, q1 = 0.0, q2 = 0.0;
-      uint32_t key = 0xffffffffu, nparts = 0;
-      if (ready) {
-        const RedSlot& rs = s_red[lane];
-        q0 = (double)rs.val[0][0] + (double)rs.val[0][1] + (double)rs.val[0][2] + (double)rs.val[0][3];
-        q1 = (double)rs.val[1][0] + (double)rs.val[1][1] + (double)rs.val[1][2] + (double)rs.val[1][3];
-        q2 = (double)rs.val[2][0] + (double)rs.val[2][1] + (double)rs.val[2][2] + (double)rs.val[2][3];
-        key = (rs.tensor << 1) | (rs.is_a & 1u);
-        nparts = rs.nparts;
-        mbar_arrive(bar_redempty + 8 * lane);  // the slot has been read
-        ++n_seen;
-      }
-      unsigned pending = __ballot_sync(0xffffffffu, ready);
-      if (pending == 0) {
+      if (!__any_sync(0xffffffffu, ready)) {
         if (end) break;
-        __nanosleep(64);
+        __nanosleep(32);
         continue;
       }
-      // Items of the same tensor and kind that completed since the last look go out as one
-      // update of the tensor's accumulators (the lowest of their lanes does it), and all such
-      // groups go out at the same time: one pair of round trips to L2 per look, however many
-      // tensors the block has chunks of.
-      const unsigned same = __match_any_sync(0xffffffffu, ready ? key : (0x80000000u | (uint32_t)lane));
+      uint32_t key = 0x80000000u | (uint32_t)lane, nparts = 0;
+      if (ready) {
+        key = (s_red[lane].tensor << 1) | s_red[lane].is_a;
+        nparts = s_red[lane].nparts;
+      }
+      const unsigned same = __match_any_sync(0xffffffffu, key);
       const bool leads = ready && (__ffs(same) - 1) == lane;
-      double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      double q[3] = {0.0, 0.0, 0.0};
+      __syncwarp();
+      if (leads) {
+        for (unsigned left = same; left != 0; left &= left - 1u) {
+          const RedSlot& rs = s_red[__ffs(left) - 1];
 #pragma unroll
-      for (int l = 0; l < S; ++l) {
-        const double b0 = __shfl_sync(0xffffffffu, q0, l), b1 = __shfl_sync(0xffffffffu, q1, l),
-                     b2 = __shfl_sync(0xffffffffu, q2, l);
-        const double w = (double)((same >> l) & 1u);  // 1.0 for the lanes of this group, else 0.0
-        a0 = fma(b0, w, a0);
-        a1 = fma(b1, w, a1);
-        a2 = fma(b2, w, a2);
+          for (int w = 0; w < 3; ++w) {
+            const float4 x = *reinterpret_cast<const float4*>(rs.val[w]);  // one value per warp of the group
+            q[w] += ((double)x.x + (double)x.y) + ((double)x.z + (double)x.w);
+          }
+        }
+      }
+      __syncwarp();
+      if (ready) {
+        mbar_arrive(bar_redempty + 8 * lane);  // the buffer has been read
+        ++n_seen;
       }
       if (leads) {
         const bool is_a = (key & 1u) != 0;
         LansCtl* ctl = P.ctl + (key >> 1);
         // A -> ||g||^2 ; B -> ||p||^2, ||update_m||^2, ||update_g||^2
         if (is_a) {
-          atomicAdd(&ctl->sumsq[0], a0);
+          atomicAdd(&ctl->sumsq[0], q[0]);
         } else {
-          atomicAdd(&ctl->sumsq[1], a0);
-          atomicAdd(&ctl->sumsq[2], a1);
-          atomicAdd(&ctl->sumsq[3], a2);
+          atomicAdd(&ctl->sumsq[1], q[0]);
+          atomicAdd(&ctl->sumsq[2], q[1]);
+          atomicAdd(&ctl->sumsq[3], q[2]);
         }
-        __threadfence();
+        fence_gpu();
         const unsigned cnt = (unsigned)__popc(same);
         const unsigned old = atomicAdd(is_a ? &ctl->arrived_a : &ctl->arrived_b, cnt);
         if (old + cnt == nparts) {
           // Every part of the tensor has been added: publish the norm(s), value and
           // "final" bit in one word each.
-          __threadfence();
+          fence_gpu();
           for (int w = is_a ? 0 : 1; w < (is_a ? 1 : 4); ++w) {
             const double total = *reinterpret_cast<volatile double*>(&ctl->sumsq[w]);
             *reinterpret_cast<volatile unsigned*>(&ctl->norm[w]) =
@@ -887,8 +941,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
                         P.wait_ns);
     if (!__all_sync(0xffffffffu, ok)) break;  // every lane of the warp leaves, or none
     const uint4 ent = s_queue[qi];
-    const uint32_t op = ent.x & 7u, slot = (ent.x >> 3) & 31u, dpar = (ent.x >> 8) & 1u, rpar = (ent.x >> 9) & 1u,
-                   opar = (ent.x >> 10) & 1u, cpar = (ent.x >> 11) & 1u;
+    const uint32_t op = ent.x & 7u, slot = (ent.x >> 3) & 31u, dpar = (ent.x >> 8) & 1u, rbuf = (ent.x >> 9) & 1u, rpar = (ent.x >> 10) & 1u;
     if (op == kOpEnd) break;
     const float cs = __uint_as_float(ent.y), ratio_m = __uint_as_float(ent.z), ratio_g = __uint_as_float(ent.w);
     // kOpCP names a tensor-memory cell, every other operation a shared-memory slot
@@ -1225,34 +1278,6 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
         }
       }
     }
-    // The bookkeeping after an operation goes to a different warp of the group each time.
-    const bool duty = (uint32_t)wig == (i & 3u);
-    if (duty) {
-      if (lane == 0) {
-        ok = ring_wait(my_done, opar, P.hdr, kErrDone, slot, P.wait_ns);
-        if (ok && op == kOpCP) {
-          // the parked chunk is in registers: its cell is free again, the item is finished
-          atomicOr(&ctrl->cell_free, 1u << cell);
-          atomicAdd(&ctrl->done_items, 1u);
-        } else if (ok) {
-          // The other three warps have let go of the slot too: its next item starts in it, or
-          // the slot is marked idle and the prefetcher starts the item when it has one.
-          if (op != kOpBP) atomicAdd(&ctrl->done_items, 1u);
-          take_next(slot);
-          if (op == kOpBP) {
-            // every warp of the group has parked its part: the parker may queue the second
-            // half as soon as the norms are final (which needs this chunk's sums, below)
-            ok = ring_wait(bar_cell + 8 * cell, cpar, P.hdr, kErrDone, 0x100u | cell, P.wait_ns);
-            if (ok) {
-              ctrl->cell_grp[cell] = (uint32_t)grp;
-              __threadfence_block();
-              atomicOr(&ctrl->cell_parked, 1u << cell);
-            }
-          }
-        }
-      }
-      if (!__shfl_sync(0xffffffffu, ok, 0)) break;
-    }
     if (publishes) {
       const float v0 = warp_sum(acc0);
       float v1 = 0.f, v2 = 0.f;
@@ -1260,11 +1285,11 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
         v1 = warp_sum(acc1);
         v2 = warp_sum(acc2);
       }
-      // the publisher has read this slot's previous sums
-      if (lane == 0) ok = ring_wait(bar_redempty + 8 * slot, rpar ^ 1u, P.hdr, kErrRing, 0x2000u | slot, P.wait_ns);
+      // the publisher has read this slot's sums before the last ones
+      if (lane == 0) ok = ring_wait(bar_redempty + 8 * (2 * slot + rbuf), rpar ^ 1u, P.hdr, kErrRing, 0x2000u | slot, P.wait_ns);
       if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       if (lane == 0) {
-        RedSlot& rs = s_red[slot];
+        RedSlot& rs = s_red[2 * slot + rbuf];
         rs.val[0][wig] = v0;
         rs.val[1][wig] = v1;
         rs.val[2][wig] = v2;
@@ -1273,7 +1298,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
           rs.is_a = (op == kOpA) ? 1u : 0u;
           rs.nparts = mt.nparts;
         }
-        mbar_arrive(bar_redfull + 8 * slot);
+        mbar_arrive(bar_redfull + 8 * (2 * slot + rbuf));
       }
     }
   }
