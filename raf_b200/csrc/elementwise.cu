@@ -541,6 +541,8 @@ template <int CAP, typename Launch>
 static int for_each_group(int k, const void* const* src, void* const* dst, const int64_t* numel, int64_t scale, int span,
                           Launch launch) {
   CopyRows<CAP> rows;
+  for (int i = 0; i < k; ++i)  // before the first launch: a refused call has done nothing
+    RAFB200_REQUIRE(numel[i] >= 0 && (numel[i] == 0 || (src[i] && dst[i])), "tensor %d of %d: NULL or of negative size", i, k);
   int n = 0;
   uint64_t spans = 0;
   for (int i = 0; i < k; ++i) {

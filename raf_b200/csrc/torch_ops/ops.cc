@@ -10,7 +10,9 @@
 
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <dlfcn.h>
@@ -58,19 +60,27 @@ int code_of(at::ScalarType t) {
   }
 }
 
-// A dense CUDA tensor on the current device, or nullptr.
-const at::Tensor* plain(PyObject* o, c10::DeviceIndex device) {
+// Tensors that stand for something else than the values at their address: fake and functional
+// ones, subclasses with a dispatch of their own, vmap's batches, lazy negation.
+const c10::DispatchKeySet kWrapped({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::Negative,
+                                    c10::DispatchKey::ZeroTensor, c10::DispatchKey::FuncTorchBatched,
+                                    c10::DispatchKey::FuncTorchGradWrapper});
+
+// A dense CUDA tensor on the current device, or nullptr.  `device` is -1 until the first CUDA tensor
+// is met: without a GPU asking for the current device throws, and tensors of the CPU are to be refused
+// by the caller's own checks.
+const at::Tensor* plain(PyObject* o, c10::DeviceIndex& device) {
   if (!THPVariable_Check(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || t.layout() != at::kStrided || !t.is_cuda() || t.device().index() != device || !t.is_contiguous())
-    return nullptr;
-  return &t;
+  if (!t.defined() || t.layout() != at::kStrided || !t.is_cuda() || t.key_set().has_any(kWrapped)) return nullptr;
+  if (device < 0) device = c10::cuda::current_device();
+  return t.device().index() == device && t.is_contiguous() ? &t : nullptr;
 }
 
-// The same outside any autograd graph.
-const at::Tensor* data_only(PyObject* o, c10::DeviceIndex device) {
+// The same outside any autograd graph, forward mode included.
+const at::Tensor* data_only(PyObject* o, c10::DeviceIndex& device) {
   const at::Tensor* t = plain(o, device);
-  return t && !t->requires_grad() ? t : nullptr;
+  return t && !t->requires_grad() && !t->_fw_grad(0).defined() ? t : nullptr;
 }
 
 void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }
@@ -95,7 +105,7 @@ at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type) {
 // sgd(x, dx, v, learning_rate, mu) -> (v1, x1)
 PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 5) return nothing();
-  const c10::DeviceIndex dev = c10::cuda::current_device();
+  c10::DeviceIndex dev = -1;
   const at::Tensor *x = data_only(a[0], dev), *dx = data_only(a[1], dev), *v = data_only(a[2], dev);
   if (!x || !dx || !v) return nothing();
   const int code = code_of(dx->scalar_type());
@@ -141,7 +151,7 @@ bool overlap(std::vector<Range>& r) {
 // launch for all of them.
 PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 3 || !PyList_CheckExact(a[0])) return nothing();
-  const c10::DeviceIndex dev = c10::cuda::current_device();
+  c10::DeviceIndex dev = -1;
   const double lr = PyFloat_AsDouble(a[1]), mu = PyFloat_AsDouble(a[2]);
   if (PyErr_Occurred()) {
     PyErr_Clear();
@@ -166,7 +176,7 @@ PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
     const at::Tensor& g = x->grad();
     if (!g.defined()) continue;
     const int c = code_of(g.scalar_type());
-    if (g.layout() != at::kStrided || !g.is_cuda() || g.device() != x->device() || !g.is_contiguous() || c < 0 ||
+    if (g.layout() != at::kStrided || !g.is_cuda() || g.device() != x->device() || !g.is_contiguous() || g.key_set().has_any(kWrapped) || c < 0 ||
         (code >= 0 && c != code) || x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat ||
         g.numel() != x->numel() || v->numel() != x->numel() || x->numel() >= (int64_t(1) << 31))
       return nothing();
@@ -211,7 +221,7 @@ struct TensorRow {
   std::vector<const at::Tensor*> t;
   std::vector<const void*> ptr;
   std::vector<int64_t> numel;
-  bool take(PyObject* seq, c10::DeviceIndex device) {
+  bool take(PyObject* seq, c10::DeviceIndex& device) {
     if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return false;
     const Py_ssize_t k = PySequence_Fast_GET_SIZE(seq);
     PyObject** items = PySequence_Fast_ITEMS(seq);
@@ -240,7 +250,7 @@ PyObject* wrapped_list(std::vector<at::Tensor>& ts) {
 PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
   static const at::ScalarType types[] = {at::kFloat, at::kHalf, at::kBFloat16};
   if (n != 3) return nothing();
-  const c10::DeviceIndex dev = c10::cuda::current_device();
+  c10::DeviceIndex dev = -1;
   TensorRow in;
   void* stream = nullptr;
   const long to = PyLong_AsLong(a[1]);
@@ -267,7 +277,7 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
 // fuse_tensor(tensors, stream) -> flat tensor
 PyObject* fuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 2) return nothing();
-  const c10::DeviceIndex dev = c10::cuda::current_device();
+  c10::DeviceIndex dev = -1;
   TensorRow in;
   void* stream = nullptr;
   if (!in.take(a[0], dev) || !stream_of(a[1], dev, &stream)) return nothing();
@@ -303,7 +313,7 @@ bool ints_of(PyObject* seq, std::vector<int64_t>* out) {
 // defuse_tensor(flat, sizes, shapes, shape_indices, stream) -> list
 PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (n != 5) return nothing();
-  const c10::DeviceIndex dev = c10::cuda::current_device();
+  c10::DeviceIndex dev = -1;
   const at::Tensor* flat = plain(a[0], dev);
   std::vector<int64_t> sizes, dims, ends, at_elem;
   void* stream = nullptr;
@@ -337,13 +347,30 @@ PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   return wrapped_list(outs);
 }
 
+using Fast = PyObject* (*)(PyObject*, PyObject* const*, Py_ssize_t);
+
+// A C++ exception (the allocator out of memory, first of all) becomes the Python exception that
+// torch raises for it; through a plain C entry it would end the process.
+template <Fast F>
+PyObject* guarded(PyObject* self, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  // under a dispatch mode torch's own calls of the slow way are what the mode gets to see
+  if (c10::impl::TorchDispatchModeTLS::any_modes_set()) return nothing();
+  return F(self, a, n);
+  END_HANDLE_TH_ERRORS
+}
+template <Fast F>
+PyCFunction fast() {
+  return reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(&guarded<F>));
+}
+
 PyMethodDef kMethods[] = {
     {"bind", bind, METH_O, "use the C ABI of the loaded library at this path"},
-    {"sgd", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd)), METH_FASTCALL, "raf.op.sgd"},
-    {"sgd_step", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(sgd_step)), METH_FASTCALL, "eager SGD, all parameters"},
-    {"group_cast", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(group_cast)), METH_FASTCALL, "raf.op.group_cast"},
-    {"fuse_tensor", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(fuse_tensor)), METH_FASTCALL, "raf.op.fuse_tensor"},
-    {"defuse_tensor", reinterpret_cast<PyCFunction>(reinterpret_cast<void*>(defuse_tensor)), METH_FASTCALL,
+    {"sgd", fast<sgd>(), METH_FASTCALL, "raf.op.sgd"},
+    {"sgd_step", fast<sgd_step>(), METH_FASTCALL, "eager SGD, all parameters"},
+    {"group_cast", fast<group_cast>(), METH_FASTCALL, "raf.op.group_cast"},
+    {"fuse_tensor", fast<fuse_tensor>(), METH_FASTCALL, "raf.op.fuse_tensor"},
+    {"defuse_tensor", fast<defuse_tensor>(), METH_FASTCALL,
      "raf.op.defuse_tensor"},
     {nullptr, nullptr, 0, nullptr}};
 

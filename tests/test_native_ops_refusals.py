@@ -1,0 +1,45 @@
+"""The native module of the operators hands everything unusual back to Python, and what its
+allocations throw arrives as torch's own exception."""
+import gc
+
+import pytest
+import torch
+
+from raf_b200 import _lib, op
+
+
+def calls(t):
+    return [lambda: op.sgd(t, t, t, 0.1, 0.9), lambda: op.group_cast([t], "float16"), lambda: op.fuse_tensor([t]),
+            lambda: op.defuse_tensor(t, [t.numel()], [t.numel()], [1])]
+
+
+@pytest.mark.parametrize("which", range(4))
+def test_cpu_tensors_are_refused(which):
+    with pytest.raises(ValueError, match="no CPU path"):
+        calls(torch.zeros(4))[which]()
+
+
+def test_null_tensors_are_refused_before_a_launch():
+    lib = _lib.load()
+    addr, n = _lib.ptr_array([4096, 0]), _lib.i64_array([8, 8])
+    at = _lib.i64_array([0, 8])
+    other = _lib.ptr_array([8192, 16384])
+    for src, dst in ((addr, other), (other, addr)):
+        assert lib.rafb200_group_cast(2, src, _lib.F32, dst, _lib.F16, n, None) == 1
+    assert lib.rafb200_fuse_tensor(2, addr, n, at, 4, 8192, None) == 1
+    assert lib.rafb200_defuse_tensor(2, addr, n, at, 4, 8192, None) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", range(4))
+def test_out_of_memory_is_torchs_exception(which):
+    gc.collect()
+    torch.cuda.empty_cache()
+    t = torch.zeros((64 << 20) + torch.cuda.memory_reserved(), device="cuda")  # no cached block holds its copy
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) / total)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            calls(t)[which]()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
