@@ -251,6 +251,18 @@ RAFB200_API int rafb200_lans_partition(int k, const int64_t* numel, int g_dtype,
 RAFB200_API int rafb200_lans_status(rafb200_tensor_list_t list, const void* workspace,
                                     float* norms_host, void* stream);
 
+/* The same update of k fp32 tensors without a tensor list, for callers that bring their tensors anew
+ * on every call (python/raf/optim/lans.py:87-99): the tables travel in the launches, up to 512
+ * tensors each.  One launch where every tensor has at most 16384 elements, else a memset and three;
+ * no block waits for another one, so there is no status to ask for.  Arithmetic as in
+ * rafb200_lans.  `step` is a host integer; host arrays of k entries, entries may be empty, the tensors must
+ * not overlap.  workspace: 16384 bytes of device memory, 16-byte aligned. */
+RAFB200_API int rafb200_lans_many(int k, const float* const* g, float* const* p, float* const* m,
+                                  float* const* v, const int64_t* numel, int step, float learning_rate,
+                                  float beta1, float beta2, float eps, int bias_correction,
+                                  float weight_decay, int grad_averaging, int mode, int normalize_grad,
+                                  float grad_scale, void* workspace, size_t workspace_bytes, void* stream);
+
 /*
  * LANS update of ONE tensor without any device allocation, by the library or by
  * the caller.  This entry point has no counterpart in the reference, whose

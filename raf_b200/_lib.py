@@ -55,6 +55,7 @@ SIGNATURES = {
     "rafb200_sgd_list": (_i, [_vp, _f, _f, _f, _f, _vp]),
     "rafb200_lans_workspace_bytes": (_sz, [_vp]),
     "rafb200_lans": (_i, [_vp, _i, _vp, _f, _f, _f, _f, _i, _f, _i, _i, _i, _f, _vp, _sz, _vp]),
+    "rafb200_lans_many": (_i, [_i, _vp, _vp, _vp, _vp, _vp, _i, _f, _f, _f, _f, _i, _f, _i, _i, _i, _f, _vp, _sz, _vp]),
     "rafb200_lans_schedule": (_i, [_i, _vp, _i, _i, _i, _i64, _i, _vp, _sz, _P(_sz)]),
     "rafb200_tensor_list_set_wait_limit": (_i, [_vp, _i]),
     "rafb200_tensor_list_set_lans_items": (_i, [_vp, _vp, _sz]),

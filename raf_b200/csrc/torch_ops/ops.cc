@@ -29,6 +29,7 @@ namespace {
 struct {
   decltype(&rafb200_sgd_to) sgd_to;
   decltype(&rafb200_sgd_many) sgd_many;
+  decltype(&rafb200_lans_many) lans_many;
   decltype(&rafb200_group_cast) group_cast;
   decltype(&rafb200_fuse_tensor) fuse_tensor;
   decltype(&rafb200_defuse_tensor) defuse_tensor;
@@ -45,6 +46,7 @@ PyObject* bind(PyObject*, PyObject* path) {
     return fn != nullptr;
   };
   if (!find(abi.sgd_to, "rafb200_sgd_to") || !find(abi.sgd_many, "rafb200_sgd_many") ||
+      !find(abi.lans_many, "rafb200_lans_many") ||
       !find(abi.group_cast, "rafb200_group_cast") || !find(abi.fuse_tensor, "rafb200_fuse_tensor") ||
       !find(abi.defuse_tensor, "rafb200_defuse_tensor"))
     return nullptr;
@@ -201,6 +203,45 @@ PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                     (float)mu, current_stream(dev));
     if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   }
+  Py_RETURN_TRUE;
+}
+
+// lans(tensors, step, learning_rate, beta1, beta2, eps, bias_correction, weight_decay, grad_averaging,
+// mode, normalize_grad) -> True: tensors = g + p + m + v, all fp32, p, m and v updated in place.
+PyObject* lans(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  if (n != 11 || !PyList_CheckExact(a[0]) || !PyLong_Check(a[1])) return nothing();
+  const Py_ssize_t count = PyList_GET_SIZE(a[0]), k = count / 4;
+  if (count == 0 || count % 4 != 0 || k > 0x7fffffff) return nothing();
+  const long step = PyLong_AsLong(a[1]), bias_correction = PyLong_AsLong(a[6]), averaging = PyLong_AsLong(a[8]),
+             mode = PyLong_AsLong(a[9]);
+  const double lr = PyFloat_AsDouble(a[2]), beta1 = PyFloat_AsDouble(a[3]), beta2 = PyFloat_AsDouble(a[4]),
+               eps = PyFloat_AsDouble(a[5]), wd = PyFloat_AsDouble(a[7]);
+  const int normalize = PyObject_IsTrue(a[10]);
+  if (PyErr_Occurred()) {
+    PyErr_Clear();
+    return nothing();
+  }
+  if (step < 1 || step > 0x7fffffff || (mode != 0 && mode != 1) || normalize < 0) return nothing();
+  c10::DeviceIndex dev = -1;
+  std::vector<float*> ptr(count);
+  std::vector<int64_t> numel(k);
+  std::vector<Range> ranges(count);
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    const at::Tensor* t = plain(PyList_GET_ITEM(a[0], i), dev);
+    if (!t || t->scalar_type() != at::kFloat || t->numel() >= (int64_t(1) << 31)) return nothing();
+    if (i < k) numel[i] = t->numel();
+    if (t->numel() != numel[i % k]) return nothing();
+    ptr[i] = static_cast<float*>(t->data_ptr());
+    const uintptr_t at_byte = reinterpret_cast<uintptr_t>(ptr[i]);
+    ranges[i] = {at_byte, at_byte + 4 * (uintptr_t)t->numel(), i >= k};
+  }
+  if (overlap(ranges)) return nothing();
+  const size_t bytes = 32 * 512;
+  c10::DataPtr workspace = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+  const int rc = abi.lans_many((int)k, ptr.data(), ptr.data() + k, ptr.data() + 2 * k, ptr.data() + 3 * k, numel.data(),
+                               (int)step, (float)lr, (float)beta1, (float)beta2, (float)eps, (int)bias_correction, (float)wd,
+                               (int)averaging, (int)mode, normalize, 1.0f, workspace.get(), bytes, current_stream(dev));
+  if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   Py_RETURN_TRUE;
 }
 
@@ -368,6 +409,7 @@ PyMethodDef kMethods[] = {
     {"bind", bind, METH_O, "use the C ABI of the loaded library at this path"},
     {"sgd", fast<sgd>(), METH_FASTCALL, "raf.op.sgd"},
     {"sgd_step", fast<sgd_step>(), METH_FASTCALL, "eager SGD, all parameters"},
+    {"lans", fast<lans>(), METH_FASTCALL, "raf.op.lans"},
     {"group_cast", fast<group_cast>(), METH_FASTCALL, "raf.op.group_cast"},
     {"fuse_tensor", fast<fuse_tensor>(), METH_FASTCALL, "raf.op.fuse_tensor"},
     {"defuse_tensor", fast<defuse_tensor>(), METH_FASTCALL,

@@ -154,24 +154,30 @@ struct LansStage1 {
   // constant: with the choice made once per chunk, the arithmetic of the elements a thread
   // holds is one straight line of code that the compiler can interleave.
   template <int MODE>
-  __device__ __forceinline__ void apply(float g, float p, float& m, float& v, float cs, float& um,
-                                        float& ug) const {
-    float sg = g * cs;
+  __device__ __forceinline__ float scaled(float g, float p, float cs) const {
+    const float sg = g * cs;
+    return MODE == 0 ? fmaf(wd, p, sg) : sg;
+  }
+  // update_m and update_g from the new m and v
+  template <int MODE>
+  __device__ __forceinline__ void directions(float sg, float p, float m, float v, float& um, float& ug) const {
+    const float r = rcp_approx(sqrt_approx(v * inv_bc2) + eps);
     if (MODE == 0) {
-      sg = fmaf(wd, p, sg);
-      m = fmaf(beta3, sg, m * beta1);
-      v = fmaf(one_minus_beta2 * sg, sg, v * beta2);
-      const float r = rcp_approx(sqrt_approx(v * inv_bc2) + eps);
       um = (m * inv_bc1) * r;
       ug = sg * r;
     } else {
-      m = fmaf(beta3, sg, m * beta1);
-      v = fmaf(one_minus_beta2 * sg, sg, v * beta2);
-      const float r = rcp_approx(sqrt_approx(v * inv_bc2) + eps);
       const float sp = wd * p;
       um = fmaf(m * inv_bc1, r, sp);
       ug = fmaf(sg, r, sp);
     }
+  }
+  template <int MODE>
+  __device__ __forceinline__ void apply(float g, float p, float& m, float& v, float cs, float& um,
+                                        float& ug) const {
+    const float sg = scaled<MODE>(g, p, cs);
+    m = fmaf(beta3, sg, m * beta1);
+    v = fmaf(one_minus_beta2 * sg, sg, v * beta2);
+    directions<MODE>(sg, p, m, v, um, ug);
   }
 };
 

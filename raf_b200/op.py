@@ -207,6 +207,12 @@ def lans(tensor_list: List[torch.Tensor], step, learning_rate, beta1, beta2, eps
     Like the reference (src/op/dialect/cuda/lans.cc:38-40) it takes fp32 tensors only;
     16-bit gradients go through :class:`TensorList` / :func:`lans_list_`.
     """
+    done = _lib.ops().lans(tensor_list, step, learning_rate, beta1, beta2, eps, bias_correction, weight_decay,
+                           grad_averaging, mode, normalize_grad)
+    if done is True:
+        return tensor_list
+    if done is not None:
+        check(done)
     n = len(tensor_list)
     if n % 4 != 0:
         raise ValueError("lans: tensor_list must hold g, p, m and v lists of equal length")

@@ -1,0 +1,76 @@
+"""raf.op.lans without a tensor list (rafb200_lans_many): one block per tensor up to 16384 elements, three
+launches above, 512 tensors a launch.  Against the oracle, at the 1e-5 that sums of squares in fp32
+allow for LANS, and against the persistent kernel, whose arithmetic is the same but for the order
+of the sums."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+from raf_b200 import _lib, op
+from tests.util import rel_err, to_numpy
+
+pytestmark = pytest.mark.gpu
+
+LISTS = {
+    "one": [1],
+    "block": [1, 3, 4, 127, 128, 4095, 4096, 4097, 16383, 16384],
+    "phases": [16385, 1, 2047, 2048, 2049, 4096],
+    "many": [5 + i % 300 for i in range(513)],
+    "many_large": [17000] + [1 + i % 40 for i in range(600)],
+    "empty_among": [0, 10, 0, 20000, 0],
+}
+
+
+def _lists(sizes, shift, seed):
+    rng = np.random.default_rng(seed)
+    host = [[(rng.standard_normal(n) * s).astype(np.float32) for n in sizes] for s in (1e-2, 0.1, 1e-3)]
+    host.append([(1e-6 * (0.5 + rng.random(n))).astype(np.float32) for n in sizes])
+
+    def place(x):  # `shift` elements past an allocation's start
+        buf = torch.zeros(x.size + shift, device="cuda")
+        buf[shift:] = torch.from_numpy(x).cuda()
+        return buf[shift:]
+
+    return host, [[place(x) for x in xs] for xs in host]
+
+
+@pytest.mark.parametrize("mode,normalize", [(1, True), (0, True), (1, False)])
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("name", list(LISTS))
+def test_lans_rows_match_oracle_and_list_kernel(name, shift, mode, normalize):
+    sizes = LISTS[name]
+    host, dev = _lists(sizes, shift, 3)
+    other = [[t.clone() for t in ts] for ts in dev]
+    args = (7, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, mode, normalize)
+    assert _lib.ops().lans(sum(dev, []), *args) is True
+    full = [i for i, n in enumerate(sizes) if n]
+    O.lans(*[[xs[i] for i in full] for xs in host], 7, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, mode, int(normalize), 1.0)
+    tl = op.TensorList(sizes, torch.float32, torch.float32)
+    tl.bind(*other)
+    op.lans_list_(tl, *args)
+    op.lans_status(tl)
+    for what in (1, 2, 3):
+        for i in full:
+            assert rel_err(to_numpy(dev[what][i]), host[what][i]) < 1e-5, (what, sizes[i])
+            assert rel_err(to_numpy(dev[what][i]), to_numpy(other[what][i])) < 1e-5, (what, sizes[i])
+
+
+def test_lans_rows_edge_values():
+    # a zero gradient (no normalisation, trust ratio 1) and a zero parameter, in both forms
+    for n in (100, 20000):
+        g, p, m, v = ([torch.zeros(n, device="cuda"), torch.full((n,), 0.5, device="cuda")] for _ in range(4))
+        hg, hp, hm, hv = ([to_numpy(x).copy() for x in xs] for xs in (g, p, m, v))
+        op.lans(g + p + m + v, 1, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, 1, True)
+        O.lans(hg, hp, hm, hv, 1, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, 1, 1, 1.0)
+        for a, b in zip(p + m + v, hp + hm + hv):
+            assert rel_err(to_numpy(a), b) < 1e-5
+
+
+def test_tied_parameters_and_device_steps_take_the_list_kernel():
+    x = [torch.ones(64, device="cuda") for _ in range(4)]
+    tied = [x[0], x[0], x[1], x[1], x[2], x[2], x[3], x[3]]
+    args = (1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, 1, True)
+    assert _lib.ops().lans(tied, 1, *args) is None
+    assert _lib.ops().lans(x, torch.ones((), device="cuda"), *args) is None
+    op.lans(x, torch.ones((), device="cuda"), *args)
