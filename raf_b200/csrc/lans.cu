@@ -136,6 +136,12 @@ __device__ __forceinline__ uint2 ld_global_v2(const void* p) {
 __device__ __forceinline__ float norm_value(unsigned bits) {
   return __uint_as_float(bits & ~kNormValid);
 }
+// A norm and its "final" bit in one word.  A norm that is no number is written out as a constant: setting the
+// sign bit of a float is compiled to a negation, and the negation of a NaN leaves the bit clear (an
+// overflowed gradient then looked like a norm that never came, and the step ended in an expired wait).
+__device__ __forceinline__ unsigned norm_word(float norm) {
+  return norm == norm ? (__float_as_uint(norm) | kNormValid) : 0xffffffffu;
+}
 
 // `step` as a 0-d fp32 device tensor (python/raf/optim/lans.py:239): the bias
 // corrections of lans.cc:100-105 (float base, int exponent, evaluated in
@@ -906,8 +912,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
           fence_gpu();
           for (int w = is_a ? 0 : 1; w < (is_a ? 1 : 4); ++w) {
             const double total = *reinterpret_cast<volatile double*>(&ctl->sumsq[w]);
-            *reinterpret_cast<volatile unsigned*>(&ctl->norm[w]) =
-                __float_as_uint(sqrtf((float)total)) | kNormValid;
+            *reinterpret_cast<volatile unsigned*>(&ctl->norm[w]) = norm_word(sqrtf((float)total));
           }
         }
       }
