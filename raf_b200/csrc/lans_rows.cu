@@ -113,6 +113,7 @@ __device__ __forceinline__ void row_stage1(const LansRow& r, int e, const LansSt
   for (int j = 0; j < kVec; ++j) {
     float um, ug;
     s1.template apply<MODE>(g.x[j], p.x[j], m.x[j], v.x[j], cs, um, ug);
+    if (e + j >= r.n) um = ug = 0.f;  // zeros past the end: 0 / (0 + eps) is no number without an eps
     acc[0] = fmaf(p.x[j], p.x[j], acc[0]);
     acc[1] = fmaf(um, um, acc[1]);
     acc[2] = fmaf(ug, ug, acc[2]);

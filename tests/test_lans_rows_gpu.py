@@ -67,6 +67,20 @@ def test_lans_rows_edge_values():
             assert rel_err(to_numpy(a), b) < 1e-5
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("name", ["block", "phases"])
+def test_lans_rows_without_eps(name, mode):
+    """eps = 0: lanes past the end of a tensor hold zeros, whose directions 0 / 0 belong to no sum."""
+    sizes = LISTS[name] + [17408, 24577]
+    host, dev = _lists(sizes, 0, 5)
+    args = (7, 1e-3, 0.9, 0.999, 0.0, 1, 0.01, 1, mode, True)
+    assert _lib.ops().lans(sum(dev, []), *args) is True
+    O.lans(*host, *args[:-1], 1, 1.0)
+    for what in (1, 2, 3):
+        for a, b in zip(dev[what], host[what]):
+            assert rel_err(to_numpy(a), b) < 1e-5, (what, b.size)
+
+
 def test_tied_parameters_and_device_steps_take_the_list_kernel():
     x = [torch.ones(64, device="cuda") for _ in range(4)]
     tied = [x[0], x[0], x[1], x[1], x[2], x[2], x[3], x[3]]
