@@ -924,9 +924,10 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
   // ================================ consumers ================================
   // Thread `gtid` of a group owns, in every chunk, the vectors of four elements at
   // q*512 + 4*gtid: 16-byte shared-memory accesses without bank conflicts, coalesced
-  // 16-byte stores.  Lanes past the end of a ragged chunk hold zeros, which add nothing
-  // to any sum.  One warp of the group (they take turns) also turns the slot over when an
-  // item's last operation is done: it starts the slot's next item from its mailbox right away.
+  // 16-byte stores.  Lanes past the end of a ragged chunk hold g = p = m = 0 and v = 1, which add nothing
+  // to any sum (with v = 0 their directions would be 0 / 0 where eps is 0).  A warp arrives on
+  // bar_done (bar_cell) once the slot's (cell's) values are in its registers; after four arrivals
+  // the turnover warp uses the slot (cell) again.
   const int grp = warp >> 2, wig = warp & 3, gtid = tid & (kGroupThreads - 1);
   Policies pol;
   pol.init();
@@ -1106,7 +1107,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
               rg[q].x[j] = in ? Elem<GT>::to_f32(gg[e + j]) : 0.f;
               rp[q].x[j] = in ? gp[e + j] : 0.f;
               rm[q].x[j] = in ? gm[e + j] : 0.f;
-              rv[q].x[j] = in ? gv[e + j] : 0.f;
+              rv[q].x[j] = in ? gv[e + j] : 1.f;
             }
           }
         }
@@ -1290,7 +1291,7 @@ __global__ void __launch_bounds__(kLansThreads, 1) lans_kernel(const LansParams 
         v1 = warp_sum(acc1);
         v2 = warp_sum(acc2);
       }
-      // the publisher has read this slot's sums before the last ones
+      // the publisher has read this buffer's sums before the last ones
       if (lane == 0) ok = ring_wait(bar_redempty + 8 * (2 * slot + rbuf), rpar ^ 1u, P.hdr, kErrRing, 0x2000u | slot, P.wait_ns);
       if (!__shfl_sync(0xffffffffu, ok, 0)) break;
       if (lane == 0) {

@@ -74,11 +74,16 @@ def test_lans_rows_without_eps(name, mode):
     sizes = LISTS[name] + [17408, 24577]
     host, dev = _lists(sizes, 0, 5)
     args = (7, 1e-3, 0.9, 0.999, 0.0, 1, 0.01, 1, mode, True)
+    other = [[t.clone() for t in ts] for ts in dev]
     assert _lib.ops().lans(sum(dev, []), *args) is True
+    tl = op.TensorList(sizes, torch.float32, torch.float32)
+    tl.bind(*other)
+    op.lans_list_(tl, *args)
+    op.lans_status(tl)
     O.lans(*host, *args[:-1], 1, 1.0)
     for what in (1, 2, 3):
-        for a, b in zip(dev[what], host[what]):
-            assert rel_err(to_numpy(a), b) < 1e-5, (what, b.size)
+        for a, c, b in zip(dev[what], other[what], host[what]):
+            assert rel_err(to_numpy(a), b) < 1e-5 and rel_err(to_numpy(c), b) < 1e-5, (what, b.size)
 
 
 def test_tied_parameters_and_device_steps_take_the_list_kernel():
