@@ -47,10 +47,13 @@ __global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE, GT>)
 // address or peer by peer at TensorDesc's symmetric offset (kept in first_chunk / nchunks) and
 // also written to the rank's local gradient block; the model-dtype copy goes into every rank's
 // parameter buffer.  The symmetric layout is 16-byte aligned and zero-padded per row block.
-// passes in flight per thread (four were measured slower: 128 registers, half the resident blocks)
+// Bound: the latency of the loads over the links, so resident blocks count: 80 registers for Adam, three
+// blocks an SM (AdamOp::vec left alone takes 96 and two blocks); SGD has 48 without a bound.  Buffers of
+// two / three "ranks" on one GPU, 44,353,792 elements, bf16: 312 / 369 us, with two blocks 354 / 431 us.
+// Passes in flight per thread: four were measured slower (128 registers, half the resident blocks).
 constexpr int kFusedUnroll = 2;
 template <int NSTATE, typename GT, typename OT, typename Op>
-__global__ void __launch_bounds__(kBlockThreads)
+__global__ void __launch_bounds__(kBlockThreads, NSTATE == 2 ? 3 : 0)
     update_list_fused_kernel(const TensorDesc* __restrict__ descs, const Item* __restrict__ items,
                              uint32_t nitems, Op op, LansFuse fu) {
   constexpr int kDT = sizeof(GT) == 4 ? RAFB200_F32 : (std::is_same<GT, __half>::value ? RAFB200_F16 : RAFB200_BF16);
