@@ -15,18 +15,18 @@ namespace rafb200 {
 // stores.  Against 8 resident blocks an SM that stride over the items (the last of 5.3 rounds was
 // 27 % full): ResNet-50 SGD, 25,557,032 elements, 87.9 -> 80.8 us, and 77.2 us (6.6 TB/s) with the
 // next step's blocks placed and their table rows read while this step's last blocks finish.
-// Adam, 44,353,792 elements with bf16 gradients: 215 -> 200 us (6.2 TB/s), with AdamOp::vec's
-// straight-line arithmetic, without which this launch shape would be slower than the old one.
-// The minimum of resident blocks is what each register count was fastest at (six blocks of the
-// fp32-gradient Adam spill: 81 against 74 us on 16 Mi elements).
+// Adam, 44,353,792 elements with bf16 gradients: 215 -> 186 us (6.7 TB/s) with AdamOp::vec's
+// straight-line arithmetic, 204 us without it (any operand outside its ranges).
+// The minimum of resident blocks is the largest without a spill: six blocks are 40 registers, with
+// which Adam spills (16-bit gradients 194 against 186 us; fp32, 16 Mi elements, 81 against 74 us).
 constexpr int kSpanUnroll = 2;
 constexpr int kSpanElems = kPassElems * kSpanUnroll;           // 2048
 constexpr int kSpansPerChunk = kChunkElems / kSpanElems;       // list items cover two spans
-template <int NSTATE, typename GT>
-constexpr int kMinBlocks = (NSTATE == 1 || sizeof(GT) == 2) ? 6 : 5;
+template <int NSTATE>
+constexpr int kMinBlocks = NSTATE == 1 ? 6 : 5;
 
 template <int NSTATE, typename GT, typename OT, typename Op>
-__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE, GT>)
+__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE>)
     update_list_kernel(const TensorDesc* __restrict__ descs, const Item* __restrict__ items, Op op) {
   Policies pol;
   pol.init();
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kBlockThreads, NSTATE == 2 ? 3 : 0)
 
 // One tensor described by value.
 template <int NSTATE, typename GT, typename OT, typename Op>
-__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE, GT>)
+__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<NSTATE>)
     update_flat_kernel(TensorDesc d, Op op) {
   Policies pol;
   pol.init();
@@ -204,7 +204,7 @@ struct Rows {
 constexpr int kMaxRows = 512;  // 16 KB of the 32 KB a launch's parameters may take
 
 template <typename GT, int CAP>
-__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<1, GT>)
+__global__ void __launch_bounds__(kBlockThreads, kMinBlocks<1>)
     sgd_rows_kernel(const __grid_constant__ Rows<CAP> rows, int k, SgdOp op) {
   Policies pol;
   pol.init();
