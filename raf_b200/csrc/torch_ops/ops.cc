@@ -365,13 +365,14 @@ PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   for (size_t i = 0; i < sizes.size(); ++i) {
     if (ends[i] < from || ends[i] > (int64_t)dims.size()) return nothing();
     int64_t numel = 1;
-    for (int64_t d = from; d < ends[i]; ++d) numel *= dims[d];
-    if (numel != sizes[i]) return nothing();
+    for (int64_t d = from; d < ends[i]; ++d)  // torch.empty refuses what 64 bits cannot count
+      if (__builtin_mul_overflow(numel, dims[d], &numel)) return nothing();
+    if (numel != sizes[i] || numel > flat->numel() - total) return nothing();
     at_elem.push_back(total);
     total += sizes[i];
     from = ends[i];
   }
-  if (sizes.empty() || total > flat->numel()) return nothing();
+  if (sizes.empty()) return nothing();
   std::vector<at::Tensor> outs;
   std::vector<void*> dst;
   outs.reserve(sizes.size());

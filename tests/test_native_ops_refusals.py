@@ -43,3 +43,16 @@ def test_out_of_memory_is_torchs_exception(which):
             calls(t)[which]()
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,shapes,indices", [
+    ([0], [1 << 32, 1 << 32], [2]),  # the product is 2^64: 0 in 64 bits
+    ([4], [(1 << 62) + 1, 4], [2]),  # 2^64 + 4
+    ([(1 << 62) + 1] * 4, [(1 << 62) + 1] * 4, [1, 2, 3, 4]),  # the sum is 2^64 + 4
+])
+def test_defuse_tensor_sizes_beyond_64_bits(sizes, shapes, indices):
+    flat = torch.zeros(8, device="cuda")
+    assert _lib.ops().defuse_tensor(flat, sizes, shapes, indices, None) is None
+    with pytest.raises(RuntimeError):  # torch.empty's, in front of any launch
+        op.defuse_tensor(flat, sizes, shapes, indices)
