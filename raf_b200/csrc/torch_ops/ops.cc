@@ -68,11 +68,12 @@ const c10::DispatchKeySet kWrapped({c10::DispatchKey::Python, c10::DispatchKey::
                                     c10::DispatchKey::ZeroTensor, c10::DispatchKey::FuncTorchBatched,
                                     c10::DispatchKey::FuncTorchGradWrapper});
 
-// A dense CUDA tensor on the current device, or nullptr.  `device` is -1 until the first CUDA tensor
+// A dense CUDA tensor on the current device (torch.Tensor or Parameter itself: what torch's own calls make
+// of a subclass is of that class), or nullptr.  `device` is -1 until the first CUDA tensor
 // is met: without a GPU asking for the current device throws, and tensors of the CPU are to be refused
 // by the caller's own checks.
 const at::Tensor* plain(PyObject* o, c10::DeviceIndex& device) {
-  if (!THPVariable_Check(o)) return nullptr;
+  if (!THPVariable_CheckExact(o)) return nullptr;
   const at::Tensor& t = THPVariable_Unpack(o);
   if (!t.defined() || t.layout() != at::kStrided || !t.is_cuda() || t.key_set().has_any(kWrapped)) return nullptr;
   if (device < 0) device = c10::cuda::current_device();

@@ -56,3 +56,16 @@ def test_defuse_tensor_sizes_beyond_64_bits(sizes, shapes, indices):
     assert _lib.ops().defuse_tensor(flat, sizes, shapes, indices, None) is None
     with pytest.raises(RuntimeError):  # torch.empty's, in front of any launch
         op.defuse_tensor(flat, sizes, shapes, indices)
+
+
+class Sub(torch.Tensor):
+    pass
+
+
+@pytest.mark.gpu
+def test_subclasses_stay_what_they_are():
+    x = torch.ones(5, device="cuda")
+    s = x.as_subclass(Sub)
+    assert all(type(t) is Sub for t in op.sgd(s, x, s, 0.1, 0.9)) and type(op.group_cast([s], "float16")[0]) is Sub
+    p = torch.nn.Parameter(x, requires_grad=False)
+    assert all(type(t) is torch.Tensor for t in _lib.ops().sgd(p, x, x, 0.1, 0.9))
