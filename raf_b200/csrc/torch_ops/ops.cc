@@ -104,6 +104,13 @@ at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type) {
   t.unsafeGetTensorImpl()->set_sizes_contiguous(sizes);
   return t;
 }
+// torch.empty_like of a dense tensor: strides of dimensions of one element are kept as they are (a 1x1
+// convolution weight in channels_last).
+at::Tensor new_like(const at::Tensor& x, at::ScalarType type) {
+  at::Tensor t = new_tensor(x.sizes(), type);
+  if (x.numel() > 0) t.unsafeGetTensorImpl()->set_sizes_and_strides(x.sizes(), x.strides());
+  return t;
+}
 
 // sgd(x, dx, v, learning_rate, mu) -> (v1, x1)
 PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
@@ -120,8 +127,8 @@ PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat || code < 0 || x->sizes() != dx->sizes() ||
       x->sizes() != v->sizes())
     return nothing();
-  at::Tensor x1 = new_tensor(x->sizes(), at::kFloat);
-  at::Tensor v1 = new_tensor(x->sizes(), at::kFloat);
+  at::Tensor x1 = new_like(*x, at::kFloat);
+  at::Tensor v1 = new_like(*v, at::kFloat);
   const int rc = abi.sgd_to(x->const_data_ptr<float>(), dx->const_data_ptr(), code, v->const_data_ptr<float>(),
                                 x1.mutable_data_ptr<float>(), v1.mutable_data_ptr<float>(), x->numel(), (float)lr, (float)mu,
                                 current_stream(dev));
@@ -307,7 +314,7 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
   outs.reserve(in.t.size());
   dst.reserve(in.t.size());
   for (const at::Tensor* x : in.t) {
-    outs.push_back(new_tensor(x->sizes(), types[to]));
+    outs.push_back(new_like(*x, types[to]));
     dst.push_back(outs.back().mutable_data_ptr());
   }
   const int rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0]->scalar_type()), dst.data(), (int)to,

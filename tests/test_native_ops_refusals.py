@@ -69,3 +69,16 @@ def test_subclasses_stay_what_they_are():
     assert all(type(t) is Sub for t in op.sgd(s, x, s, 0.1, 0.9)) and type(op.group_cast([s], "float16")[0]) is Sub
     p = torch.nn.Parameter(x, requires_grad=False)
     assert all(type(t) is torch.Tensor for t in _lib.ops().sgd(p, x, x, 0.1, 0.9))
+
+
+@pytest.mark.gpu
+def test_strides_of_single_elements_are_kept():
+    x = torch.empty_strided((64, 32, 1, 1), (32, 1, 32, 32), device="cuda").zero_()  # channels_last
+    y = torch.zeros(64, 32, 1, 1, device="cuda")
+    v1, x1 = op.sgd(x, y, y, 0.1, 0.9)
+    assert x.is_contiguous() and x1.stride() == x.clone().stride() and v1.stride() == y.clone().stride()
+    assert op.group_cast([x], "float16")[0].stride() == torch.empty_like(x).stride()
+    for shape in ((0,), (0, 3), (), (1,), (1, 0, 2)):
+        e = torch.zeros(shape, device="cuda")
+        assert op.group_cast([e], "float16")[0].stride() == torch.empty_like(e).stride()
+        assert op.sgd(e, e, e, 0.1, 0.9)[0].shape == e.shape
