@@ -10,6 +10,7 @@
 
 #include <ATen/core/Tensor.h>
 #include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/core/GradMode.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -80,10 +81,10 @@ const at::Tensor* plain(PyObject* o, c10::DeviceIndex& device) {
   return t.device().index() == device && t.is_contiguous() ? &t : nullptr;
 }
 
-// The same outside any autograd graph, forward mode included.
+// The same where the result belongs to no autograd graph, forward mode included.
 const at::Tensor* data_only(PyObject* o, c10::DeviceIndex& device) {
   const at::Tensor* t = plain(o, device);
-  return t && !t->requires_grad() && !t->_fw_grad(0).defined() ? t : nullptr;
+  return t && !(t->requires_grad() && c10::GradMode::is_enabled()) && !t->_fw_grad(0).defined() ? t : nullptr;
 }
 
 void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDAStream(device).stream(); }

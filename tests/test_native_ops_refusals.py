@@ -82,3 +82,14 @@ def test_strides_of_single_elements_are_kept():
         e = torch.zeros(shape, device="cuda")
         assert op.group_cast([e], "float16")[0].stride() == torch.empty_like(e).stride()
         assert op.sgd(e, e, e, 0.1, 0.9)[0].shape == e.shape
+
+
+@pytest.mark.gpu
+def test_sgd_on_parameters():
+    """Without grad mode the result is data; with it, what torch's own clone makes of a parameter."""
+    p, x = torch.nn.Parameter(torch.ones(5, device="cuda")), torch.full((5,), 2.0, device="cuda")
+    with torch.no_grad():
+        v1, x1 = _lib.ops().sgd(p, x, x, 0.5, 0.5)
+    assert not x1.requires_grad and v1.tolist() == [3.0] * 5 and x1.tolist() == [-0.5] * 5
+    assert _lib.ops().sgd(p, x, x, 0.5, 0.5) is None
+    assert op.sgd(p, x, x, 0.5, 0.5)[1].grad_fn is not None
