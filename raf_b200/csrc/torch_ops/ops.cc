@@ -91,6 +91,18 @@ void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDA
 
 PyObject* nothing() { Py_RETURN_NONE; }
 
+// The GIL is released while a function allocates and launches: either may block (the allocator frees its
+// cache, a launch queue is full) on something that another Python thread has to bring about.  A call costs
+// 0.05 us more.  Tensors that are looked at meanwhile are the caller's arguments or copies: a list may
+// lose its own to another thread.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+  NoGil() = default;
+  NoGil(const NoGil&) = delete;
+  NoGil& operator=(const NoGil&) = delete;
+};
+
 // torch.empty on the current device, from torch's caching allocator: 0.5 us where the dispatched
 // form takes 1.3 us, and the list operators make up to hundreds of tensors a call.
 at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type) {
@@ -128,11 +140,16 @@ PyObject* sgd(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (x->scalar_type() != at::kFloat || v->scalar_type() != at::kFloat || code < 0 || x->sizes() != dx->sizes() ||
       x->sizes() != v->sizes())
     return nothing();
-  at::Tensor x1 = new_like(*x, at::kFloat);
-  at::Tensor v1 = new_like(*v, at::kFloat);
-  const int rc = abi.sgd_to(x->const_data_ptr<float>(), dx->const_data_ptr(), code, v->const_data_ptr<float>(),
-                                x1.mutable_data_ptr<float>(), v1.mutable_data_ptr<float>(), x->numel(), (float)lr, (float)mu,
-                                current_stream(dev));
+  at::Tensor x1, v1;
+  int rc;
+  {
+    NoGil released;
+    x1 = new_like(*x, at::kFloat);
+    v1 = new_like(*v, at::kFloat);
+    rc = abi.sgd_to(x->const_data_ptr<float>(), dx->const_data_ptr(), code, v->const_data_ptr<float>(),
+                    x1.mutable_data_ptr<float>(), v1.mutable_data_ptr<float>(), x->numel(), (float)lr, (float)mu,
+                    current_stream(dev));
+  }
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   PyObject* out = PyTuple_New(2);
   if (!out) return nullptr;
@@ -208,8 +225,12 @@ PyObject* sgd_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   if (overlap(ranges)) return nothing();  // tied parameters: one after the other, as the loop does
   if (!xs.empty()) {
-    const int rc = abi.sgd_many((int)xs.size(), xs.data(), gs.data(), code, vs.data(), numel.data(), (float)lr,
-                                    (float)mu, current_stream(dev));
+    int rc;
+    {
+      NoGil released;
+      rc = abi.sgd_many((int)xs.size(), xs.data(), gs.data(), code, vs.data(), numel.data(), (float)lr, (float)mu,
+                        current_stream(dev));
+    }
     if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   }
   Py_RETURN_TRUE;
@@ -246,10 +267,14 @@ PyObject* lans(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   if (overlap(ranges)) return nothing();
   const size_t bytes = 32 * 512;
-  c10::DataPtr workspace = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
-  const int rc = abi.lans_many((int)k, ptr.data(), ptr.data() + k, ptr.data() + 2 * k, ptr.data() + 3 * k, numel.data(),
-                               (int)step, (float)lr, (float)beta1, (float)beta2, (float)eps, (int)bias_correction, (float)wd,
-                               (int)averaging, (int)mode, normalize, 1.0f, workspace.get(), bytes, current_stream(dev));
+  int rc;
+  {
+    NoGil released;
+    c10::DataPtr workspace = c10::cuda::CUDACachingAllocator::get()->allocate(bytes);
+    rc = abi.lans_many((int)k, ptr.data(), ptr.data() + k, ptr.data() + 2 * k, ptr.data() + 3 * k, numel.data(), (int)step,
+                       (float)lr, (float)beta1, (float)beta2, (float)eps, (int)bias_correction, (float)wd, (int)averaging,
+                       (int)mode, normalize, 1.0f, workspace.get(), bytes, current_stream(dev));
+  }
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   Py_RETURN_TRUE;
 }
@@ -268,7 +293,7 @@ bool stream_of(PyObject* o, c10::DeviceIndex device, void** stream) {
 
 // A non-empty list or tuple of dense CUDA tensors of one type: addresses and element counts.
 struct TensorRow {
-  std::vector<const at::Tensor*> t;
+  std::vector<at::Tensor> t;
   std::vector<const void*> ptr;
   std::vector<int64_t> numel;
   bool take(PyObject* seq, c10::DeviceIndex& device) {
@@ -280,8 +305,8 @@ struct TensorRow {
     numel.reserve(k);
     for (Py_ssize_t i = 0; i < k; ++i) {
       const at::Tensor* x = plain(items[i], device);
-      if (!x || x->scalar_type() != (i ? t[0] : x)->scalar_type()) return false;
-      t.push_back(x);
+      if (!x || x->scalar_type() != (i ? t[0] : *x).scalar_type()) return false;
+      t.push_back(*x);
       ptr.push_back(x->const_data_ptr());
       numel.push_back(x->numel());
     }
@@ -308,18 +333,22 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyErr_Clear();
     return nothing();
   }
-  if (to < 0 || to > 2 || !in.take(a[0], dev) || code_of(in.t[0]->scalar_type()) < 0 || !stream_of(a[2], dev, &stream))
+  if (to < 0 || to > 2 || !in.take(a[0], dev) || code_of(in.t[0].scalar_type()) < 0 || !stream_of(a[2], dev, &stream))
     return nothing();
   std::vector<at::Tensor> outs;
   std::vector<void*> dst;
   outs.reserve(in.t.size());
   dst.reserve(in.t.size());
-  for (const at::Tensor* x : in.t) {
-    outs.push_back(new_like(*x, types[to]));
-    dst.push_back(outs.back().mutable_data_ptr());
+  int rc;
+  {
+    NoGil released;
+    for (const at::Tensor& x : in.t) {
+      outs.push_back(new_like(x, types[to]));
+      dst.push_back(outs.back().mutable_data_ptr());
+    }
+    rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0].scalar_type()), dst.data(), (int)to,
+                        in.numel.data(), stream);
   }
-  const int rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0]->scalar_type()), dst.data(), (int)to,
-                                in.numel.data(), stream);
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   return wrapped_list(outs);
 }
@@ -337,9 +366,14 @@ PyObject* fuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
     at_elem[i] = total;
     total += in.numel[i];
   }
-  at::Tensor flat = new_tensor({total}, in.t[0]->scalar_type());
-  const int rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(),
-                                 (int)in.t[0]->element_size(), flat.mutable_data_ptr(), stream);
+  at::Tensor flat;
+  int rc;
+  {
+    NoGil released;
+    flat = new_tensor({total}, in.t[0].scalar_type());
+    rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(), (int)in.t[0].element_size(),
+                         flat.mutable_data_ptr(), stream);
+  }
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   return THPVariable_Wrap(std::move(flat));
 }
@@ -387,13 +421,17 @@ PyObject* defuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   outs.reserve(sizes.size());
   dst.reserve(sizes.size());
   from = 0;
-  for (size_t i = 0; i < sizes.size(); ++i) {
-    outs.push_back(new_tensor(at::IntArrayRef(dims.data() + from, (size_t)(ends[i] - from)), flat->scalar_type()));
-    dst.push_back(outs.back().mutable_data_ptr());
-    from = ends[i];
+  int rc;
+  {
+    NoGil released;
+    for (size_t i = 0; i < sizes.size(); ++i) {
+      outs.push_back(new_tensor(at::IntArrayRef(dims.data() + from, (size_t)(ends[i] - from)), flat->scalar_type()));
+      dst.push_back(outs.back().mutable_data_ptr());
+      from = ends[i];
+    }
+    rc = abi.defuse_tensor((int)sizes.size(), dst.data(), sizes.data(), at_elem.data(), (int)flat->element_size(),
+                           flat->const_data_ptr(), stream);
   }
-  const int rc = abi.defuse_tensor((int)sizes.size(), dst.data(), sizes.data(), at_elem.data(),
-                                   (int)flat->element_size(), flat->const_data_ptr(), stream);
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
   return wrapped_list(outs);
 }

@@ -1,6 +1,8 @@
 """The native module of the operators hands everything unusual back to Python, and what its
 allocations throw arrives as torch's own exception."""
 import gc
+import threading
+import time
 
 import pytest
 import torch
@@ -93,3 +95,22 @@ def test_sgd_on_parameters():
     assert not x1.requires_grad and v1.tolist() == [3.0] * 5 and x1.tolist() == [-0.5] * 5
     assert _lib.ops().sgd(p, x, x, 0.5, 0.5) is None
     assert op.sgd(p, x, x, 0.5, 0.5)[1].grad_fn is not None
+
+
+@pytest.mark.gpu
+def test_a_full_launch_queue_stalls_no_other_thread():
+    x = torch.ones(5, device="cuda")
+    _lib.ops().sgd(x, x, x, 0.1, 0.9)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(1_000_000_000)  # half a second; what follows waits behind it
+    start = last = time.perf_counter()
+    caller = threading.Thread(target=lambda: [_lib.ops().sgd(x, x, x, 0.1, 0.9) for _ in range(3000)])
+    caller.start()
+    longest = 0.0
+    while caller.is_alive():
+        time.sleep(1e-3)
+        now = time.perf_counter()
+        longest, last = max(longest, now - last), now
+    caller.join()
+    assert last - start > 0.3, "the queue never filled"
+    assert longest < 0.15
