@@ -6,7 +6,10 @@ library cannot be loaded, importing this module raises.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.environ.get("RAFB200_LIB") or os.path.join(HERE, "libraf_b200.so")  # an installed copy elsewhere
@@ -122,19 +125,33 @@ _lib = None
 _ops = None
 
 
+class _GeneralWay:
+    """Stands in for the native module where it cannot be built or loaded: every call is handed back."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def ops():
-    """The native module of the operators (csrc/torch_ops/ops.cc), built first when missing."""
+    """The native module of the operators (csrc/torch_ops/ops.cc), built first when missing.  Without it
+    the operators run the same kernels through ctypes."""
     global _ops
     if _ops is None:
+        from . import build as _build
+
         load()  # libraf_b200.so and torch are in the process before the module links to them
-        if not os.path.exists(os.path.join(HERE, "_ops.so")):
-            from . import build as _build
-
-            _build.build_ops()
-        from . import _ops as mod
-
-        mod.bind(LIB_PATH)
-        _ops = mod
+        try:
+            path = _build.ops_path()
+            if not os.path.exists(path):
+                _build.build_ops()
+            loader = importlib.machinery.ExtensionFileLoader(__package__ + "._ops", path)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+            loader.exec_module(mod)
+            mod.bind(LIB_PATH)
+            _ops = mod
+        except (ImportError, OSError, RuntimeError) as exc:
+            warnings.warn(f"raf_b200._ops is not available, operators take the slower way through ctypes: {exc}")
+            _ops = _GeneralWay()
     return _ops
 
 

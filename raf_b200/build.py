@@ -10,8 +10,9 @@ into ``raf_b200/libraf_b200_glue.so``, so that the glue is type-checked and can
 be driven on fake tensors by the tests.  Inside a RAF tree the same file is
 compiled against RAF's own headers instead.
 
-Last comes ``raf_b200/_ops.so`` (``csrc/torch_ops/ops.cc``), the CPython module through which the
-operators reach the library without a detour over ctypes.
+Last comes ``raf_b200._ops`` (``csrc/torch_ops/ops.cc``), the CPython module through which the
+operators reach the library without a detour over ctypes.  Its file name holds the versions of Python and
+torch it was built for, whose object layouts it is compiled against.
 """
 from __future__ import annotations
 
@@ -19,13 +20,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_obj")
 LIB = os.path.join(HERE, "libraf_b200.so")
-OPS_LIB = os.path.join(HERE, "_ops.so")
 GLUE_LIB = os.path.join(HERE, "libraf_b200_glue.so")
 COMPAT = os.path.join(CSRC, "raf_compat")
 
@@ -98,32 +99,44 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     return LIB
 
 
-def build_ops(force: bool = False) -> str:
-    """ops.cc, a CPython module over torch's C++ API -> _ops.so (host code only)."""
-    src = os.path.join(CSRC, "torch_ops", "ops.cc")
-    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "raf_b200.h")))
-    if not force and os.path.exists(OPS_LIB) and os.path.getmtime(OPS_LIB) >= newest:
-        return OPS_LIB
-    import sysconfig
+def ops_path() -> str:
+    """The file of raf_b200._ops for this Python and this torch."""
+    import torch
 
+    versions = f"{sysconfig.get_config_var('SOABI')}-torch-{torch.__version__}"
+    return os.path.join(HERE, "_ops." + "".join(c if c.isalnum() or c in "-." else "_" for c in versions) + ".so")
+
+
+def build_ops(force: bool = False) -> str:
+    """ops.cc, a CPython module over torch's C++ API (host code only)."""
+    src, out = os.path.join(CSRC, "torch_ops", "ops.cc"), ops_path()
+    newest = max(os.path.getmtime(src), os.path.getmtime(os.path.join(HERE, "..", "include", "raf_b200.h")))
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= newest:
+        return out
     import torch
     from torch.utils import cpp_extension
 
+    part = f"{out}.{os.getpid()}"  # several ranks may build at first use: each puts a whole file in place
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-Wall",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            "-I" + sysconfig.get_paths()["include"], "-I/usr/local/cuda/include"]
     for d in cpp_extension.include_paths():
         cmd += ["-isystem", d]
-    cmd += ["-o", OPS_LIB, src]
+    cmd += ["-o", part, src]
     for d in cpp_extension.library_paths():
         cmd += ["-L" + d, "-Wl,-rpath," + d]
     cmd += ["-ldl", "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu",
             "-lc10_cuda", "-lc10"]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
-        raise RuntimeError("building raf_b200._ops failed")
-    return OPS_LIB
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode != 0:
+            sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
+            raise RuntimeError("building raf_b200._ops failed")
+        os.replace(part, out)
+    finally:
+        if os.path.exists(part):
+            os.remove(part)
+    return out
 
 
 def build_glue(nvcc: str, force: bool = False) -> str:

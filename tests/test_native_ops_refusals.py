@@ -1,13 +1,14 @@
 """The native module of the operators hands everything unusual back to Python, and what its
 allocations throw arrives as torch's own exception."""
 import gc
+import os
 import threading
 import time
 
 import pytest
 import torch
 
-from raf_b200 import _lib, op
+from raf_b200 import _lib, build, op
 
 
 def calls(t):
@@ -30,6 +31,55 @@ def test_null_tensors_are_refused_before_a_launch():
         assert lib.rafb200_group_cast(2, src, _lib.F32, dst, _lib.F16, n, None) == 1
     assert lib.rafb200_fuse_tensor(2, addr, n, at, 4, 8192, None) == 1
     assert lib.rafb200_defuse_tensor(2, addr, n, at, 4, 8192, None) == 1
+
+
+def test_operators_work_without_the_native_module(monkeypatch, tmp_path):
+    monkeypatch.setattr(_lib, "_ops", None)
+    monkeypatch.setattr(build, "ops_path", lambda: str(tmp_path / "missing.so"))
+    monkeypatch.setattr(build.subprocess, "run", lambda *a, **k: (_ for _ in ()).throw(FileNotFoundError("no g++")))
+    with pytest.warns(UserWarning, match="no g\\+\\+"):
+        assert _lib.ops().sgd(1, 2, 3, 4, 5) is None
+    with pytest.raises(ValueError, match="no CPU path"):
+        calls(torch.zeros(4))[0]()
+
+
+def test_a_build_puts_a_whole_module_in_place_or_none(monkeypatch, tmp_path):
+    out = tmp_path / "ops.so"
+    out.write_text("the one before")
+    os.utime(out, (0, 0))
+    monkeypatch.setattr(build, "ops_path", lambda: str(out))
+
+    def link(cmd, **kw):  # dies half way
+        with open(cmd[cmd.index("-o") + 1], "w") as f:
+            f.write("half")
+        assert out.read_text() == "the one before"
+        return build.subprocess.CompletedProcess(cmd, code, "", "")
+
+    monkeypatch.setattr(build.subprocess, "run", link)
+    code = 1
+    with pytest.raises(RuntimeError):
+        build.build_ops()
+    assert out.read_text() == "the one before" and len(list(tmp_path.iterdir())) == 1
+    code = 0
+    build.build_ops()
+    assert out.read_text() == "half" and len(list(tmp_path.iterdir())) == 1
+
+
+def test_the_module_is_named_after_the_versions_it_is_built_for(monkeypatch):
+    before = build.ops_path()
+    monkeypatch.setattr(torch, "__version__", "9.9")
+    assert build.ops_path() != before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("which", range(4))
+def test_without_the_native_module_the_results_are_the_same(monkeypatch, which):
+    t = torch.arange(5000, device="cuda", dtype=torch.float32) / 7
+    want = calls(t)[which]()
+    monkeypatch.setattr(_lib, "_ops", _lib._GeneralWay())
+    got = calls(t)[which]()
+    for a, b in zip(got, want):
+        assert a.dtype == b.dtype and torch.equal(a, b)
 
 
 @pytest.mark.gpu
