@@ -840,13 +840,18 @@ static int step_impl(rafb200_zero_t z, const rafb200_hyper* h, int step, void* c
     std::vector<int64_t> bytes;
   };
   constexpr size_t kSmallBytes = 256 << 10;
-  auto device_view = [](const void* host_ptr) -> void* {  // of page-locked memory; NULL for other memory
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, host_ptr) != cudaSuccess) {
+  // Device address of a piece of page-locked memory; NULL for other memory, and where the piece reaches
+  // past what is page-locked: a copy reports that, a kernel would fault.
+  auto device_view = [](const void* host_ptr, size_t bytes) -> void* {
+    cudaPointerAttributes first, last;
+    if (cudaPointerGetAttributes(&first, host_ptr) != cudaSuccess ||
+        cudaPointerGetAttributes(&last, static_cast<const char*>(host_ptr) + bytes - 1) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }
-    return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
+    const bool whole = first.type == cudaMemoryTypeHost && last.type == cudaMemoryTypeHost && first.devicePointer &&
+                       static_cast<char*>(last.devicePointer) == static_cast<char*>(first.devicePointer) + (bytes - 1);
+    return whole ? first.devicePointer : nullptr;
   };
   // Pieces that follow one another in host AND device memory, inside ranges the caller declared to
   // be single allocations, travel as one copy: a caller that keeps its gradients (parameters) in
@@ -867,7 +872,7 @@ static int step_impl(rafb200_zero_t z, const rafb200_hyper* h, int step, void* c
     if (bytes == 0 && src) return RAFB200_OK;  // an empty piece; src NULL: end of the run
     if (r.bytes) {
       const bool in = kind == cudaMemcpyHostToDevice;
-      void* mapped = small && r.bytes < kSmallBytes ? device_view(in ? r.src : r.dst) : nullptr;
+      void* mapped = small && r.bytes < kSmallBytes ? device_view(in ? r.src : r.dst, r.bytes) : nullptr;
       if (mapped) {
         small->src.push_back(in ? mapped : r.src);
         small->dst.push_back(in ? r.dst : mapped);
