@@ -313,6 +313,8 @@ def defuse_tensor(data, sizes, shapes, shape_indices, stream=None):
         assert outs[-1].numel() == n
         offsets.append(off)
         off += n
+    if off > data.numel():
+        raise ValueError(f"defuse_tensor: sizes hold {off} elements, data {data.numel()}")
     check(_lib.load().rafb200_defuse_tensor(
         len(outs), _lib.ptr_array([t.data_ptr() for t in outs]), _lib.i64_array(sizes),
         _lib.i64_array(offsets), data.element_size(), data.data_ptr(), stream_ptr(stream)))

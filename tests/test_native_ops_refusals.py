@@ -164,3 +164,9 @@ def test_a_full_launch_queue_stalls_no_other_thread():
     caller.join()
     assert last - start > 0.3, "the queue never filled"
     assert longest < 0.15
+
+
+@pytest.mark.gpu
+def test_defuse_tensor_of_too_few_elements():
+    with pytest.raises(ValueError, match="9 elements"):
+        op.defuse_tensor(torch.zeros(8, device="cuda"), [4, 5], [4, 5], [1, 2])
