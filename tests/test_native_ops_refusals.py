@@ -170,3 +170,68 @@ def test_a_full_launch_queue_stalls_no_other_thread():
 def test_defuse_tensor_of_too_few_elements():
     with pytest.raises(ValueError, match="9 elements"):
         op.defuse_tensor(torch.zeros(8, device="cuda"), [4, 5], [4, 5], [1, 2])
+
+
+def native(t):
+    """Every function of the module on one tensor, as the operators call it."""
+    ops, n = _lib.ops(), t.numel()
+    return [ops.sgd(t, t, t, 0.1, 0.9), ops.sgd_step([(t, t)], 0.1, 0.9), ops.group_cast([t], 1, None),
+            ops.lans([t, t, t, t], 1, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, 1, True), ops.fuse_tensor([t], None),
+            ops.defuse_tensor(t, [n], [n], [1], None)]
+
+
+def test_cpu_and_fake_tensors_are_handed_back():
+    from torch._subclasses.fake_tensor import FakeTensorMode
+
+    with FakeTensorMode():
+        fake = torch.empty(4, device="cuda")
+    for t in (torch.zeros(4), fake):
+        t.grad = torch.zeros_like(t)
+        assert native(t) == [None] * 6
+    with pytest.raises(ValueError, match="no CPU path"):
+        op.lans([torch.zeros(4)] * 4, 1, 1e-3, 0.9, 0.999, 1e-6, 1, 0.01, 1, 1, True)
+
+
+@pytest.mark.gpu
+def test_tensors_that_stand_for_others_are_handed_back():
+    """Under a dispatch mode, inside torch.func's transforms, with a lazy negation, as efficient zeros: no
+    function looks at the address."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    x = torch.ones(3, 4, device="cuda")
+    seen = []
+
+    def look(t):
+        seen.append(native(t))
+        return t.sum()
+
+    torch.func.vmap(look)(x)
+    torch.func.grad(look)(x)
+    torch.func.functionalize(look)(x)
+    look(torch._neg_view(torch.ones(4, device="cuda")))
+    look(torch._efficientzerotensor(4, device="cuda"))
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    y = torch.ones(4, device="cuda")
+    y.grad = torch.ones(4, device="cuda")
+    with Mode():
+        seen.append(native(y))
+    assert seen == [[None] * 6] * 6
+    assert y.tolist() == [1.0] * 4
+
+
+@pytest.mark.gpu
+def test_autograd_and_forward_mode_take_torchs_calls():
+    import torch.autograd.forward_ad as fwd
+
+    x = torch.ones(4, device="cuda")
+    with fwd.dual_level():
+        dual = fwd.make_dual(x, x)
+        assert _lib.ops().sgd(dual, x, x, 0.1, 0.9) is None
+        assert fwd.unpack_dual(op.sgd(dual, x, x, 0.1, 0.9)[1]).tangent is not None
+    for i in range(3):
+        args = [x.clone().requires_grad_(j == i) for j in range(3)]
+        assert _lib.ops().sgd(*args, 0.1, 0.9) is None
