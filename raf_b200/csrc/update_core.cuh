@@ -59,14 +59,17 @@ __device__ __forceinline__ float div_by(float a, float b, float y) {
   q = fmaf(fmaf(-b, q, a), y, q);
   return fmaf(fmaf(-b, q, a), y, q);
 }
-// RN(1/b): one Newton step on the hardware's approximation; equal to __frcp_rn for every one of
-// the 2^23 significands, at exponents -60 .. 60 (compared exhaustively on the device).
+// RN(1/b): one step of Newton's method for 1/y - b, y + y * (1 - b * y) with the bracket in one rounding, on
+// the hardware's approximation.  That it rounds correctly is a property of that approximation:
+// tests/test_adam_arithmetic_gpu.py compares every one of the 2^23 significands, at exponents
+// -60 .. 60, with __frcp_rn.
 __device__ __forceinline__ float rcp_rn(float b) {
   const float y = rcp_approx(b);
   return fmaf(fmaf(-b, y, 1.0f), y, y);
 }
-// RN(sqrt(x)) by one Newton step on x * rsqrt(x); equal to __fsqrt_rn for every float from 2^-100
-// to 2^100 (compared exhaustively on the device).  x must not be zero.
+// RN(sqrt(x)): one step of Newton's method for g^2 - x, g + (x - g * g) / (2 g) with the bracket in one rounding, from
+// g = x * y and 1 / (2 g) = y / 2, y the hardware's approximation of 1 / sqrt(x).  Compared with
+// __fsqrt_rn for every float from 2^-100 to 2^100 by the same test.  x must not be zero.
 __device__ __forceinline__ float sqrt_rn(float x) {
   const float y = rsqrt_approx(x);
   const float g = mul(x, y), h = mul(0.5f, y);
