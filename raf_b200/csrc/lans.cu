@@ -209,11 +209,6 @@ __device__ __forceinline__ void tma_load_1d(uint32_t dst, const void* src, uint3
       "l"(src), "r"(bytes), "r"(bar), "l"(policy)
       : "memory");
 }
-// Orders this thread's earlier generic-proxy accesses to shared memory before later
-// accesses of the async proxy (the next bulk copy into the same slot).
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
 
 // ---- tensor memory as a scratchpad ------------------------------------------------------
 // 32x32b accesses: the 32 threads of a warp address the 32 lanes of the warp's own quarter
@@ -1365,8 +1360,8 @@ int lans_a_elems(int g_dtype) { return g_dtype == RAFB200_F32 ? kLansAElems32 : 
 // How many chunks of one tensor may wait on chip at the same time, for a grid with
 // `cells_total` cells (blocks x kLansCells): five eighths.  Every block - the parked items are
 // dealt out evenly - then keeps cells for the tensors before and after a large one, whose
-// stage 1 overlaps the wait for the large tensor's norms (measured on the BERT-large list:
-// 2.20 ms at 5/8, 2.25 ms at 4/5, 2.27 ms at 3/8).
+// stage 1 overlaps the wait for the large tensor's norms (measured on the BERT-large list: 2.06 ms at
+// 5/8, 2.10 at 1/2, 2.11 at 3/4, 2.12 at 4/5, 2.13 at 3/8, 2.14 at 7/8; its shard of eight 250 - 253 us at all).
 uint32_t lans_park_cap(int64_t cells_total) {
   const int64_t cap = cells_total * 5 / 8;
   return (uint32_t)(cap < 0 ? 0 : cap);

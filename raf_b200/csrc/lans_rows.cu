@@ -27,8 +27,10 @@ bool pointers_aligned(const void* g, int g_dtype, const void* p, const void* m, 
 
 constexpr int kRowUnroll = 2;
 constexpr int kRowSpan = kPassElems * kRowUnroll;  // 2048 elements per block of the three-launch form
-// A call of the one-launch form took 7.7 us at 1000 elements a tensor, 10.9 at 8192 and 14.1 at 16384;
-// the memset and three launches took 10.6 to 19 us between 16385 and 262144 elements (host-bound, so it varies).
+// Device time of a call, one launch against a memset and three.  One to eight tensors: 7.5 us at 1000 elements, 10 at
+// 8192, 13.1 to 14 at 16384 against 10.4 from 16385 on, so up to 3.6 us are lost above 8192.  31 tensors: 13.8
+// against 12.3.  148: 14.4 against 19.0, and 12.4 us of host time less a call.  400: 52 against 51 (21 at 1000).  The
+// line lies where the many tensors of a network still gain; one by the number of tensors would be better for few.
 constexpr int kBlockElems = 16384;
 constexpr int kOneBlockThreads = 1024;
 constexpr int kLansMaxRows = 512;  // 20 KB of the 32 KB a launch's parameters may take

@@ -232,35 +232,4 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Sums N values per thread over the block; result valid in every thread.
-// `smem` needs N * (blockDim.x/32) floats.  Contains two __syncthreads().
-template <int N>
-__device__ __forceinline__ void block_sum(float (&v)[N], float* smem) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-#pragma unroll
-  for (int i = 0; i < N; ++i) v[i] = warp_sum(v[i]);
-  if (lane == 0) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) smem[i * nwarp + warp] = v[i];
-  }
-  __syncthreads();
-#pragma unroll
-  for (int i = 0; i < N; ++i) {
-    float s = 0.f;
-    for (int w = 0; w < nwarp; ++w) s += smem[i * nwarp + w];
-    v[i] = s;
-  }
-  __syncthreads();
-}
-
-// ---- flags ---------------------------------------------------------------
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
 }  // namespace rafb200
