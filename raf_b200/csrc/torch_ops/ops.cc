@@ -92,9 +92,8 @@ void* current_stream(c10::DeviceIndex device) { return c10::cuda::getCurrentCUDA
 PyObject* nothing() { Py_RETURN_NONE; }
 
 // The GIL is released while a function allocates and launches: either may block (the allocator frees its
-// cache, a launch queue is full) on something that another Python thread has to bring about.  A call costs
-// 0.05 us more.  Tensors that are looked at meanwhile are the caller's arguments or copies: a list may
-// lose its own to another thread.
+// cache, a launch queue is full) on something that another Python thread has to bring about.  Tensors that
+// are looked at meanwhile are the caller's arguments or held by the call.
 struct NoGil {
   PyThreadState* state = PyEval_SaveThread();
   ~NoGil() { PyEval_RestoreThread(state); }
@@ -291,11 +290,19 @@ bool stream_of(PyObject* o, c10::DeviceIndex device, void** stream) {
   return false;
 }
 
-// A non-empty list or tuple of dense CUDA tensors of one type: addresses and element counts.
+// A non-empty list or tuple of dense CUDA tensors of one type: addresses and element counts.  The items are
+// held by references of this call (made and given up under the GIL): another thread may change the list.
 struct TensorRow {
-  std::vector<at::Tensor> t;
+  std::vector<const at::Tensor*> t;
   std::vector<const void*> ptr;
   std::vector<int64_t> numel;
+  std::vector<PyObject*> held;
+  TensorRow() = default;
+  TensorRow(const TensorRow&) = delete;
+  TensorRow& operator=(const TensorRow&) = delete;
+  ~TensorRow() {
+    for (PyObject* o : held) Py_DECREF(o);
+  }
   bool take(PyObject* seq, c10::DeviceIndex& device) {
     if (!PyList_CheckExact(seq) && !PyTuple_CheckExact(seq)) return false;
     const Py_ssize_t k = PySequence_Fast_GET_SIZE(seq);
@@ -303,10 +310,12 @@ struct TensorRow {
     t.reserve(k);
     ptr.reserve(k);
     numel.reserve(k);
+    held.reserve(k);
     for (Py_ssize_t i = 0; i < k; ++i) {
       const at::Tensor* x = plain(items[i], device);
-      if (!x || x->scalar_type() != (i ? t[0] : *x).scalar_type()) return false;
-      t.push_back(*x);
+      if (!x || x->scalar_type() != (i ? t[0] : x)->scalar_type()) return false;
+      held.push_back(Py_NewRef(items[i]));
+      t.push_back(x);
       ptr.push_back(x->const_data_ptr());
       numel.push_back(x->numel());
     }
@@ -333,7 +342,7 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
     PyErr_Clear();
     return nothing();
   }
-  if (to < 0 || to > 2 || !in.take(a[0], dev) || code_of(in.t[0].scalar_type()) < 0 || !stream_of(a[2], dev, &stream))
+  if (to < 0 || to > 2 || !in.take(a[0], dev) || code_of(in.t[0]->scalar_type()) < 0 || !stream_of(a[2], dev, &stream))
     return nothing();
   std::vector<at::Tensor> outs;
   std::vector<void*> dst;
@@ -342,11 +351,11 @@ PyObject* group_cast(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int rc;
   {
     NoGil released;
-    for (const at::Tensor& x : in.t) {
-      outs.push_back(new_like(x, types[to]));
+    for (const at::Tensor* x : in.t) {
+      outs.push_back(new_like(*x, types[to]));
       dst.push_back(outs.back().mutable_data_ptr());
     }
-    rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0].scalar_type()), dst.data(), (int)to,
+    rc = abi.group_cast((int)in.t.size(), in.ptr.data(), code_of(in.t[0]->scalar_type()), dst.data(), (int)to,
                         in.numel.data(), stream);
   }
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
@@ -370,8 +379,8 @@ PyObject* fuse_tensor(PyObject*, PyObject* const* a, Py_ssize_t n) {
   int rc;
   {
     NoGil released;
-    flat = new_tensor({total}, in.t[0].scalar_type());
-    rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(), (int)in.t[0].element_size(),
+    flat = new_tensor({total}, in.t[0]->scalar_type());
+    rc = abi.fuse_tensor((int)in.t.size(), in.ptr.data(), in.numel.data(), at_elem.data(), (int)in.t[0]->element_size(),
                          flat.mutable_data_ptr(), stream);
   }
   if (rc != RAFB200_OK) return PyLong_FromLong(rc);
