@@ -120,7 +120,8 @@ at::Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type) {
 // convolution weight in channels_last).
 at::Tensor new_like(const at::Tensor& x, at::ScalarType type) {
   at::Tensor t = new_tensor(x.sizes(), type);
-  if (x.numel() > 0) t.unsafeGetTensorImpl()->set_sizes_and_strides(x.sizes(), x.strides());
+  if (x.strides() != t.strides() && x.numel() > 0)  // setting them takes 0.03 us, which 48 tensors show
+    t.unsafeGetTensorImpl()->set_sizes_and_strides(x.sizes(), x.strides());
   return t;
 }
 
