@@ -15,8 +15,9 @@ namespace rafb200 {
 // stores.  Against 8 resident blocks an SM that stride over the items (the last of 5.3 rounds was
 // 27 % full): ResNet-50 SGD, 25,557,032 elements, 87.9 -> 80.8 us, and 77.2 us (6.6 TB/s) with the
 // next step's blocks placed and their table rows read while this step's last blocks finish.
-// Adam, 44,353,792 elements with bf16 gradients: 215 -> 186 us (6.7 TB/s) with AdamOp::vec's
-// straight-line arithmetic, 204 us without it (any operand outside its ranges).
+// Adam, one tensor of 44,353,792 elements with bf16 gradients: 215 -> 186 us (6.7 TB/s) with AdamOp::vec's
+// straight-line arithmetic, 204 us without it (any operand outside its ranges); 194 us as the 292 tensors
+// of a shard of GPT-2-medium.
 // The minimum of resident blocks is the largest without a spill: six blocks are 40 registers, with
 // which Adam spills (16-bit gradients 194 against 186 us; fp32, 16 Mi elements, 81 against 74 us).
 constexpr int kSpanUnroll = 2;
