@@ -1461,7 +1461,7 @@ std::vector<uint32_t> partition_lans_items(const std::vector<Item>& sched, int g
   uint32_t at = 0;
   for (int hb = 0; hb < 2 * grid; ++hb) {
     out[hb] = at;
-    // Each list has its own prefetcher warp and its own half of the block's tensor-memory
+    // Each list has its own prefetcher and turnover warp and its own half of the block's
     // cells.  Its parked items carry their running number among them (modulo 2^11, far more
     // than are ever in flight) in the top bits of the chunk word; chunk indices stay below
     // 2^21.  Cells are handed out by these numbers.
